@@ -1,4 +1,5 @@
-"""ctypes binding of ``libnvfp4_b200.so`` (the C ABI in ``include/nvfp4_b200.h``).
+"""ctypes binding of ``libnvfp4_b200.so`` (the C ABI in ``include/nvfp4_b200.h``), and the native
+module that passes torch tensors to it without going through ctypes (``csrc/torch_binding.cpp``).
 
 There is no fallback: if the library is missing or a call fails, an exception is raised.
 """
@@ -150,6 +151,23 @@ def load() -> ctypes.CDLL:
     lib.nvfp4_version.restype = c_char_p
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The module ``_native.so``: the operator's entry points on torch tensors."""
+    global _native
+    if _native is None:
+        load()
+        import torch  # noqa: F401  (its libraries have to be in the process first)
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise ImportError(f"_native.so is missing or does not fit this torch ({e}): build it with `python -m nvfp4_gemm_b200.build`") from e
+        _native = module
+    return _native
 
 
 def check(rc: int) -> None:

@@ -1,7 +1,7 @@
-"""Ahead-of-time build of the CUDA library (``python -m nvfp4_gemm_b200.build``).
+"""Ahead-of-time build of the CUDA library and the torch binding (``python -m nvfp4_gemm_b200.build``).
 
-Compiles ``csrc/nvfp4_api.cu`` for sm_100a into ``libnvfp4_b200.so`` next to this file.
-nvcc cross-compiles without a GPU.  Nothing is JIT-compiled at call time (the reference
+Compiles ``csrc/nvfp4_api.cu`` for sm_100a into ``libnvfp4_b200.so`` and ``csrc/torch_binding.cpp``
+(host code only) into ``_native.so`` next to this file.  nvcc cross-compiles without a GPU.  Nothing is JIT-compiled at call time (the reference
 builds at import with ``load_inline``, s_128t.py:587-602).
 """
 from __future__ import annotations
@@ -10,11 +10,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 SRC = PKG_DIR / "csrc" / "nvfp4_api.cu"
 LIB = PKG_DIR / "libnvfp4_b200.so"
+HEADER = PKG_DIR.parent / "include" / "nvfp4_b200.h"
+BINDING_SRC = PKG_DIR / "csrc" / "torch_binding.cpp"
+BINDING = PKG_DIR / "_native.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -32,27 +36,45 @@ def find_nvcc() -> str:
 
 
 def sources() -> list[Path]:
-    return [SRC, *sorted((PKG_DIR / "csrc").glob("*.cuh")), PKG_DIR.parent / "include" / "nvfp4_b200.h"]
+    return [SRC, *sorted((PKG_DIR / "csrc").glob("*.cuh")), HEADER]
+
+
+def _newer(target: Path, inputs: list[Path]) -> bool:
+    return target.exists() and all(s.stat().st_mtime <= target.stat().st_mtime for s in inputs)
 
 
 def needs_build() -> bool:
-    if not LIB.exists():
-        return True
-    t = LIB.stat().st_mtime
-    return any(s.stat().st_mtime > t for s in sources())
+    return not _newer(LIB, sources()) or not _newer(BINDING, [BINDING_SRC, HEADER])
+
+
+def _replace(target: Path, cmd: list[str], verbose: bool) -> None:
+    tmp = target.with_suffix(".so.building")
+    cmd = [*cmd, "-o", str(tmp)]
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    subprocess.check_call(cmd)
+    os.replace(tmp, target)       # a reader never sees a half-written library
+
+
+def _build_binding(verbose: bool) -> None:
+    import torch
+    torch_dir = Path(torch.__file__).resolve().parent
+    cuda_home = Path(find_nvcc()).resolve().parent.parent
+    includes = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include", cuda_home / "include",
+                Path(sysconfig.get_paths()["include"])]
+    # (torch's own libraries are in the process when the module is loaded: torch is imported first)
+    _replace(BINDING, ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                       f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                       *[f for i in includes for f in ("-isystem", str(i))], str(BINDING_SRC),
+                       f"-L{PKG_DIR}", "-l:libnvfp4_b200.so", f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
+                       "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    if not force and not needs_build():
-        return LIB
-    tmp = LIB.with_suffix(".so.building")
-    cmd = [find_nvcc(), *NVCC_FLAGS, "-o", str(tmp), str(SRC)]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-        print(" ".join(cmd), file=sys.stderr)
-    subprocess.check_call(cmd)
-    os.replace(tmp, LIB)       # a reader never sees a half-written library
+    if force or not _newer(LIB, sources()):
+        _replace(LIB, [find_nvcc(), *(["-Xptxas", "-v"] if verbose else []), *NVCC_FLAGS, str(SRC)], verbose)
+    if force or not _newer(BINDING, [BINDING_SRC, HEADER]):
+        _build_binding(verbose)
     return LIB
 
 

@@ -1,6 +1,6 @@
-// C ABI of the library (declared in include/nvfp4_b200.h): argument validation, tensor-map
-// cache, per-device scratch, kernel selection and launch.  No allocation, tensor-map encoding
-// or synchronisation happens on the steady-state path of nvfp4_gemm / nvfp4_gemv.
+// C ABI of the library (declared in include/nvfp4_b200.h): argument validation, tensor maps,
+// per-device scratch, kernel selection and launch.  No allocation or synchronisation happens on the
+// steady-state path of nvfp4_gemm / nvfp4_gemv.
 #include "../../include/nvfp4_b200.h"
 
 #include <atomic>
@@ -10,7 +10,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <vector>
 
 #include "gemm_sm100.cuh"
 #include "gemv_sm100.cuh"
@@ -45,6 +44,7 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+// What a tensor map is encoded from.
 struct MapKey {
     const void* ptr;
     uint64_t dims[4];
@@ -53,11 +53,6 @@ struct MapKey {
     int dtype;
     int rank;
     int swizzle;
-    bool operator==(const MapKey& o) const { return std::memcmp(this, &o, sizeof(MapKey)) == 0; }
-};
-struct MapEntry {
-    MapKey key;
-    CUtensorMap map;
 };
 
 constexpr int kMaxCtas = 160;                                          // persistent CTAs (one per SM; a B200 has 148)
@@ -83,21 +78,36 @@ struct DeviceCtx {
     int* status_host = nullptr;
     int* status_dev = nullptr;
     size_t scratch_bytes = 0;
+    std::atomic<bool> scratch_ready{false};   // scratch and counters are allocated and cleared
     int max_pairs = -1;  // CTA pairs that can be co-resident (cluster occupancy), queried once
-    std::vector<MapEntry> maps;
     bool smem_attr_set[24] = {};
 };
 
 std::mutex g_mutex;
-DeviceCtx* g_ctx[64] = {nullptr};
-EncodeTiledFn g_encode = nullptr;
+std::atomic<DeviceCtx*> g_ctx[64];
+std::atomic<EncodeTiledFn> g_encode{nullptr};
+
+int find_encode(EncodeTiledFn* out) {
+    *out = g_encode.load(std::memory_order_acquire);
+    if (*out) return NVFP4_OK;
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
+    if (!fn || qres != cudaDriverEntryPointSuccess)
+        return fail(NVFP4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    *out = reinterpret_cast<EncodeTiledFn>(fn);
+    g_encode.store(*out, std::memory_order_release);
+    return NVFP4_OK;
+}
 
 int get_ctx(DeviceCtx** out) {
     int dev = -1;
     CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return fail(NVFP4_ERR_CUDA, "unexpected device ordinal %d", dev);
+    *out = g_ctx[dev].load(std::memory_order_acquire);
+    if (*out) return NVFP4_OK;
     std::lock_guard<std::mutex> lock(g_mutex);
-    if (!g_ctx[dev]) {
+    if (!g_ctx[dev].load()) {
         cudaDeviceProp prop;
         CUDA_TRY(cudaGetDeviceProperties(&prop, dev));
         DeviceCtx* c = new DeviceCtx();
@@ -107,23 +117,16 @@ int get_ctx(DeviceCtx** out) {
         CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->status_host), sizeof(int), cudaHostAllocMapped));
         *c->status_host = 0;
         CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->status_dev), c->status_host, 0));
-        g_ctx[dev] = c;
+        g_ctx[dev].store(c, std::memory_order_release);
     }
-    if (!g_encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-        if (!fn || qres != cudaDriverEntryPointSuccess)
-            return fail(NVFP4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-        g_encode = reinterpret_cast<EncodeTiledFn>(fn);
-    }
-    *out = g_ctx[dev];
+    *out = g_ctx[dev].load();
     return NVFP4_OK;
 }
 
 int ensure_scratch(DeviceCtx* c) {
+    if (c->scratch_ready.load(std::memory_order_acquire)) return NVFP4_OK;
     std::lock_guard<std::mutex> lock(g_mutex);
-    if (c->scratch) return NVFP4_OK;
+    if (c->scratch_ready.load()) return NVFP4_OK;
     // Partial-tile slots need no initialisation (they are written before they are read); the
     // per-tile counters must be zero between launches.
     CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&c->scratch), kStreamSets * kScratchBytes));
@@ -131,6 +134,7 @@ int ensure_scratch(DeviceCtx* c) {
     CUDA_TRY(cudaMemset(c->counters, 0, kStreamSets * kMaxCtas * sizeof(int)));
     CUDA_TRY(cudaDeviceSynchronize());
     c->scratch_bytes = kStreamSets * (kScratchBytes + kMaxCtas * sizeof(int));
+    c->scratch_ready.store(true, std::memory_order_release);
     return NVFP4_OK;
 }
 
@@ -171,33 +175,24 @@ int scratch_set_for(DeviceCtx* c, cudaStream_t stream, int* set) {
                 kStreamSets, c->device);
 }
 
-// Tensor maps are cached by (pointer, extents, strides, box): re-encoding four maps per call,
-// as the reference does (s_128t.py:569-577), costs more than a short GEMM.
-int get_map(DeviceCtx* c, const MapKey& key, CUtensorMap* out) {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    for (const MapEntry& e : c->maps)
-        if (e.key == key) {
-            *out = e.map;
-            return NVFP4_OK;
-        }
-    MapEntry e;
-    std::memset(&e, 0, sizeof(e));
-    e.key = key;
-    cuuint64_t dims[4] = {key.dims[0], key.dims[1], key.dims[2], key.dims[3]};
-    cuuint64_t strides[3] = {key.strides[0], key.strides[1], key.strides[2]};
-    cuuint32_t box[4] = {key.box[0], key.box[1], key.box[2], key.box[3]};
-    cuuint32_t elem[4] = {1, 1, 1, 1};
-    CUresult r = g_encode(&e.map, static_cast<CUtensorMapDataType>(key.dtype), key.rank, const_cast<void*>(key.ptr), dims,
-                          strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, static_cast<CUtensorMapSwizzle>(key.swizzle),
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+// Encodes a tensor map into caller storage.  Every call encodes its four or five maps anew, like the
+// reference (s_128t.py:569-577): one takes the CPU 49 ns, less than finding it in a table of a few
+// hundred under a lock, and a caller whose buffers are new pays no more.
+int encode_map(const MapKey& key, CUtensorMap* out) {
+    EncodeTiledFn encode = nullptr;
+    if (int rc = find_encode(&encode)) return rc;
+    const cuuint64_t dims[4] = {key.dims[0], key.dims[1], key.dims[2], key.dims[3]};
+    const cuuint64_t strides[3] = {key.strides[0], key.strides[1], key.strides[2]};
+    const cuuint32_t box[4] = {key.box[0], key.box[1], key.box[2], key.box[3]};
+    const cuuint32_t elem[4] = {1, 1, 1, 1};
+    const CUresult r = encode(out, static_cast<CUtensorMapDataType>(key.dtype), key.rank, const_cast<void*>(key.ptr), dims, strides, box, elem,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, static_cast<CUtensorMapSwizzle>(key.swizzle), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return fail(NVFP4_ERR_CUDA, "cuTensorMapEncodeTiled failed (CUresult %d) rank %d dims {%llu,%llu,%llu,%llu} strides {%llu,%llu,%llu}",
                     static_cast<int>(r), key.rank, (unsigned long long)dims[0], (unsigned long long)dims[1],
                     (unsigned long long)dims[2], (unsigned long long)dims[3], (unsigned long long)strides[0],
                     (unsigned long long)strides[1], (unsigned long long)strides[2]);
-    if (c->maps.size() >= 256) c->maps.erase(c->maps.begin());
-    c->maps.push_back(e);
-    *out = e.map;
     return NVFP4_OK;
 }
 
@@ -550,22 +545,22 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
     const uint64_t a_bs = p->l > 1 ? static_cast<uint64_t>(p->a_batch_stride) : static_cast<uint64_t>(p->a_row_stride) * p->m;
     const uint64_t b_bs = p->l > 1 ? static_cast<uint64_t>(p->b_batch_stride) : static_cast<uint64_t>(p->b_row_stride) * p->n;
     const uint64_t c_bs = p->l > 1 ? static_cast<uint64_t>(p->c_batch_stride) * 2 : static_cast<uint64_t>(p->c_row_stride) * 2 * p->m;
-    if (int rc = get_map(c, make_key(p->a, kbytes, p->m, p->l, p->a_row_stride, a_bs, kBKBytes, kBM, CU_TENSOR_MAP_DATA_TYPE_UINT8),
+    if (int rc = encode_map(make_key(p->a, kbytes, p->m, p->l, p->a_row_stride, a_bs, kBKBytes, kBM, CU_TENSOR_MAP_DATA_TYPE_UINT8),
                          &g.tma_a)) return rc;
-    if (int rc = get_map(c, make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, bn / cg, CU_TENSOR_MAP_DATA_TYPE_UINT8),
+    if (int rc = encode_map(make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, bn / cg, CU_TENSOR_MAP_DATA_TYPE_UINT8),
                          &g.tma_b)) return rc;
-    if (int rc = get_map(c, make_sf_key(p->sfa_perm, p->m, p->k, p->l, p->sfa_perm_batch_stride, 1), &g.tma_sfa)) return rc;
-    if (int rc = get_map(c, make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, bn / 128), &g.tma_sfb)) return rc;
+    if (int rc = encode_map(make_sf_key(p->sfa_perm, p->m, p->k, p->l, p->sfa_perm_batch_stride, 1), &g.tma_sfa)) return rc;
+    if (int rc = encode_map(make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, bn / 128), &g.tma_sfb)) return rc;
     g.n_peer = n_peers;
     for (int i = 0; i < n_peers; ++i) g.c_peer[i] = static_cast<__half*>(c_peers[i]);
     if (epilogue >= 2 && p->c) {
-        if (int rc = get_map(c, make_key(p->c, p->n, p->m, p->l, static_cast<uint64_t>(p->c_row_stride) * 2, c_bs, 64, 32,
+        if (int rc = encode_map(make_key(p->c, p->n, p->m, p->l, static_cast<uint64_t>(p->c_row_stride) * 2, c_bs, 64, 32,
                                          CU_TENSOR_MAP_DATA_TYPE_FLOAT16),
                              &g.tma_c)) return rc;
         if (n_peers > 0 && n_peers <= peer_tma_limit()) {
             g.peer_tma = 1;
             for (int i = 0; i < n_peers; ++i)
-                if (int rc = get_map(c, make_key(c_peers[i], p->n, p->m, p->l, static_cast<uint64_t>(p->c_row_stride) * 2, c_bs, 64, 32,
+                if (int rc = encode_map(make_key(c_peers[i], p->n, p->m, p->l, static_cast<uint64_t>(p->c_row_stride) * 2, c_bs, 64, 32,
                                                  CU_TENSOR_MAP_DATA_TYPE_FLOAT16),
                                      &g.tma_c_peer[i])) return rc;
         }
@@ -597,9 +592,9 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
         g.tiles_m = (p->m + kBM - 1) / kBM;
         g.tiles_n = p->n / bn;
         g.total_units = g.tiles_m * g.tiles_n * p->l * g.k_tiles;
-        if (int rc = get_map(c, make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, bn, CU_TENSOR_MAP_DATA_TYPE_UINT8),
+        if (int rc = encode_map(make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, bn, CU_TENSOR_MAP_DATA_TYPE_UINT8),
                              &g.tma_b)) return rc;
-        if (int rc = get_map(c, make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, bn / 128), &g.tma_sfb)) return rc;
+        if (int rc = encode_map(make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, bn / 128), &g.tma_sfb)) return rc;
         if (epi) {
             if (bn == 128 && ks == 2) return launch_gemm_splitk<128, 6, 0, 2, true>(c, 16, g, stream, "gemm_splitk2_n128_s6_epilogue");
             return fail(NVFP4_ERR_UNSUPPORTED, "the extended epilogue is built for split_k 1 and 2");
@@ -988,7 +983,8 @@ size_t nvfp4_scratch_bytes(void) {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     std::lock_guard<std::mutex> lock(g_mutex);
-    return g_ctx[dev] ? g_ctx[dev]->scratch_bytes : 0;
+    const DeviceCtx* c = g_ctx[dev].load();
+    return c ? c->scratch_bytes : 0;
 }
 
 int nvfp4_plan_units(int total_units, int grid, int cta, int* begin, int* end, int* first_tile_slot, int k_tiles) {
@@ -1060,7 +1056,7 @@ void nvfp4_shutdown(void) {
     int prev = -1;
     cudaGetDevice(&prev);
     for (int d = 0; d < 64; ++d) {
-        DeviceCtx* c = g_ctx[d];
+        DeviceCtx* c = g_ctx[d].exchange(nullptr);
         if (!c) continue;
         cudaSetDevice(d);
         cudaDeviceSynchronize();
@@ -1068,7 +1064,6 @@ void nvfp4_shutdown(void) {
         if (c->counters) cudaFree(c->counters);
         if (c->status_host) cudaFreeHost(c->status_host);
         delete c;
-        g_ctx[d] = nullptr;
     }
     if (prev >= 0) cudaSetDevice(prev);
 }
@@ -1099,7 +1094,6 @@ struct StaticScratch {
 };
 StaticScratch g_static[64];
 std::mutex g_static_mutex;
-EncodeTiledFn g_static_encode = nullptr;
 
 int static_scratch_setup(int dev, StaticScratch** out) {
     std::lock_guard<std::mutex> lock(g_static_mutex);
@@ -1117,28 +1111,7 @@ int static_scratch_setup(int dev, StaticScratch** out) {
                                       GemmSmem<1, 128, 4, false, 64>::kDynamicBytes));
         st.ready = true;
     }
-    if (!g_static_encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-        if (!fn || qres != cudaDriverEntryPointSuccess)
-            return fail(NVFP4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-        g_static_encode = reinterpret_cast<EncodeTiledFn>(fn);
-    }
     *out = &st;
-    return NVFP4_OK;
-}
-
-// Encodes a tensor map into caller storage (no cache: nothing is kept on the heap).
-int encode_map_inplace(const MapKey& key, CUtensorMap* out) {
-    cuuint64_t dims[4] = {key.dims[0], key.dims[1], key.dims[2], key.dims[3]};
-    cuuint64_t strides[3] = {key.strides[0], key.strides[1], key.strides[2]};
-    cuuint32_t box[4] = {key.box[0], key.box[1], key.box[2], key.box[3]};
-    cuuint32_t elem[4] = {1, 1, 1, 1};
-    CUresult r = g_static_encode(out, static_cast<CUtensorMapDataType>(key.dtype), key.rank, const_cast<void*>(key.ptr), dims,
-                                 strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, static_cast<CUtensorMapSwizzle>(key.swizzle),
-                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(NVFP4_ERR_CUDA, "cuTensorMapEncodeTiled failed (CUresult %d)", static_cast<int>(r));
     return NVFP4_OK;
 }
 
@@ -1194,10 +1167,10 @@ int nvfp4_gemm_static_scratch(const nvfp4_problem* p, int workers, void* stream_
     const uint64_t kbytes = static_cast<uint64_t>(p->k) / 2;
     const uint64_t a_bs = p->l > 1 ? static_cast<uint64_t>(p->a_batch_stride) : static_cast<uint64_t>(p->a_row_stride) * p->m;
     const uint64_t b_bs = p->l > 1 ? static_cast<uint64_t>(p->b_batch_stride) : static_cast<uint64_t>(p->b_row_stride) * p->n;
-    if (int rc = encode_map_inplace(make_key(p->a, kbytes, p->m, p->l, p->a_row_stride, a_bs, kBKBytes, kBM, CU_TENSOR_MAP_DATA_TYPE_UINT8), &g.tma_a)) return rc;
-    if (int rc = encode_map_inplace(make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, bn, CU_TENSOR_MAP_DATA_TYPE_UINT8), &g.tma_b)) return rc;
-    if (int rc = encode_map_inplace(make_sf_key(p->sfa_perm, p->m, p->k, p->l, p->sfa_perm_batch_stride, 1), &g.tma_sfa)) return rc;
-    if (int rc = encode_map_inplace(make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, 1), &g.tma_sfb)) return rc;
+    if (int rc = encode_map(make_key(p->a, kbytes, p->m, p->l, p->a_row_stride, a_bs, kBKBytes, kBM, CU_TENSOR_MAP_DATA_TYPE_UINT8), &g.tma_a)) return rc;
+    if (int rc = encode_map(make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, bn, CU_TENSOR_MAP_DATA_TYPE_UINT8), &g.tma_b)) return rc;
+    if (int rc = encode_map(make_sf_key(p->sfa_perm, p->m, p->k, p->l, p->sfa_perm_batch_stride, 1), &g.tma_sfa)) return rc;
+    if (int rc = encode_map(make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, 1), &g.tma_sfb)) return rc;
 
     int grid = workers > 0 ? workers : kStaticMaxWorkers;
     if (grid > st->num_sms) grid = st->num_sms;
