@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
 #include "quantize.cuh"
 
 namespace nvfp4 {
@@ -157,94 +158,117 @@ __global__ void __launch_bounds__(256) scales_from_permuted_kernel(const uint8_t
 
 // NVFP4 quantiser (the step before the matmul): fp16 / bf16 [rows][K] -> packed e2m1 + one e4m3
 // scale per 16 elements, scale = RN(max|x| / 6), element = RN(x / scale) saturated to +-6.
-// Work unit: 128 rows x 256 columns (one row block of the permuted scale layout x 4 of its atoms),
-// taken in turn by a grid of resident CTAs of 256 threads.  A thread owns 64 consecutive elements of
-// a row = four scale blocks = one 4-byte unit of both scale layouts: 128 bytes in (eight 16-byte
-// loads, all in flight before the first block is worked on; four neighbouring threads cover 512
-// bytes of a row), 32 bytes of codes and the 4-byte word of plain scales out.  The permuted scales
-// of the unit -- 4 atoms of 512 bytes, contiguous in memory -- are collected in shared memory and
-// written as whole 16-byte pieces (written from the threads' rows they would be 4-byte pieces
-// scattered over the atoms: 10 % of the run time); rows of the block that do not exist are written
-// as zero scales.
-// kWide: every output address is aligned for the wide stores (16 bytes for the codes and the
-// permuted scales, 4 bytes for the plain scale words); otherwise 8-byte and single-byte stores.
-constexpr int kQuantGroups = 4;   // 64-element groups (= scale atoms) along K per work unit
-template <bool BF16, bool kWide>
-__global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const void* __restrict__ x, uint8_t* __restrict__ packed,
-                                                             uint8_t* __restrict__ sf_plain, uint8_t* __restrict__ sf_perm, int rows,
-                                                             int k, long long x_row_stride, long long packed_row_stride,
-                                                             long long sf_plain_row_stride) {
-    __shared__ uint32_t staged[2][kQuantGroups][129];   // [unit parity][atom][word of the atom = (row % 32) * 4 + row / 32], padded
-    const int groups_per_row = k / 64;
-    const int units_k = (groups_per_row + kQuantGroups - 1) / kQuantGroups;
-    const long long units = static_cast<long long>((rows + 127) / 128) * units_k;
-    const int g = threadIdx.x & (kQuantGroups - 1);
-    int parity = 0;
-    for (long long unit = blockIdx.x; unit < units; unit += gridDim.x, parity ^= 1) {
-        const int row_block = static_cast<int>(unit / units_k);
-        const int unit_k = static_cast<int>(unit - static_cast<long long>(row_block) * units_k);
-        const int grp = unit_k * kQuantGroups + g;
+//
+// Bound by memory traffic (2 bytes in, 0.5625 or 0.625 out per element).  A lane takes one scale
+// block: 32 bytes in by one load, 8 bytes of codes and a scale byte out, and a warp 32 neighbouring
+// blocks of a row, so that every access of a warp is one contiguous piece (1024, 256 and 32 bytes; a
+// lane that takes 64 elements of a row touches 32 cache lines per load instead, 123 us on bf16
+// 8192 x 28672).  Four lanes put their scales together into the 4-byte word that both scale layouts
+// have.  A CTA of eight warps covers 8 * R rows x 512 columns; a warp asks for its R rows first of all.
+// Measured (us, bf16, graph replay, inputs beyond L2), R = 1 / 2 / 4 / 8:
+//   8192 x 28672   108.2 / 104.4 / 101.0 / 129.4   (R = 4: 6.1 TB/s)
+//   8192 x 8192     32.5 /  31.7 /  31.5 /  39.8
+//   4096 x 7168     15.2 /  15.1 /  15.8 /  21.7
+//   2048 x 7168      8.6 /   8.8 /   9.9 /  13.6
+//   128 x 7168       2.2 /   2.6 /   3.2 /   5.6
+// More rows in flight per warp help as long as there are CTAs enough to even out the end of the
+// launch; units of a whole 128-row block, with the scales collected in shared memory and written as
+// 16-byte pieces, were slower than either (129.7 and 25.6 us on 8192 and 4096 rows).
+// kWide: every address is aligned for the wide accesses (32 bytes for x, 4 for the scales); otherwise
+// 16-byte loads, and single bytes of scales.
+constexpr int kQuantCols = 512;    // columns per CTA: 32 scale blocks, 8 scale atoms
+struct QuantizeParams {
+    const uint8_t* x;
+    uint8_t* packed;
+    uint8_t* sf_plain;   // or null
+    uint8_t* sf_perm;    // or null
+    int rows, k;
+    long long x_row_stride, packed_row_stride, sf_plain_row_stride;   // bytes
+};
+template <bool kWide>
+__device__ __forceinline__ void load_block16(const uint8_t* src, uint32_t (&w)[8]) {
+    if (kWide) {
+        asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src));
+    } else {
+        const uint4 a = __ldcs(reinterpret_cast<const uint4*>(src)), b = __ldcs(reinterpret_cast<const uint4*>(src) + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    }
+}
+// Sixteen fp16 / bf16 values -> eight bytes of codes and the scale byte.
+template <bool BF16>
+__device__ __forceinline__ uint32_t quantize_words(const uint32_t (&w)[8], uint32_t (&codes)[2]) {
+    float v[16], amax;
+    if (BF16) {
+        __nv_bfloat162 top = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
 #pragma unroll
-        for (int it = 0; it < 128 * kQuantGroups / 256; ++it) {
-            const int r = it * (256 / kQuantGroups) + threadIdx.x / kQuantGroups;   // row inside the block
-            const long long row = static_cast<long long>(row_block) * 128 + r;
-            uint32_t scales = 0u;
-            if (row < rows && grp < groups_per_row) {
-                const uint8_t* src = reinterpret_cast<const uint8_t*>(static_cast<const uint16_t*>(x) + row * x_row_stride + grp * 64);
-                uint4 in[8];
+        for (int j = 1; j < 8; ++j) top = __hmax2_nan(top, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[j])));
+        const uint32_t t = *reinterpret_cast<const uint32_t*>(&top);
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(amax) : "f"(__uint_as_float(t << 16)), "f"(__uint_as_float(t & 0xffff0000u)));
 #pragma unroll
-                for (int b = 0; b < 8; ++b) in[b] = __ldcs(reinterpret_cast<const uint4*>(src) + b);
-                uint32_t codes[8];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const uint32_t w[8] = {in[2 * b].x, in[2 * b].y, in[2 * b].z, in[2 * b].w, in[2 * b + 1].x, in[2 * b + 1].y, in[2 * b + 1].z, in[2 * b + 1].w};
-                    float v[16];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if (BF16) {
-                            v[2 * j] = __uint_as_float(w[j] << 16);
-                            v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-                        } else {
-                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-                            v[2 * j] = f.x;
-                            v[2 * j + 1] = f.y;
-                        }
-                    }
-                    uint32_t out[2];
-                    const uint32_t sf_byte = quantize_block16(v, out);
-                    codes[2 * b] = out[0];
-                    codes[2 * b + 1] = out[1];
-                    scales |= sf_byte << (8 * b);
-                }
-                uint8_t* dst = packed + row * packed_row_stride + grp * 32;
-                if (kWide) {
-                    *reinterpret_cast<uint4*>(dst) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
-                    *reinterpret_cast<uint4*>(dst + 16) = make_uint4(codes[4], codes[5], codes[6], codes[7]);
-                    if (sf_plain) *reinterpret_cast<uint32_t*>(sf_plain + row * sf_plain_row_stride + grp * 4) = scales;
-                } else {
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        *reinterpret_cast<uint2*>(dst + 8 * b) = make_uint2(codes[2 * b], codes[2 * b + 1]);
-                        if (sf_plain) sf_plain[row * sf_plain_row_stride + grp * 4 + b] = static_cast<uint8_t>(scales >> (8 * b));
-                    }
-                }
-            }
-            staged[parity][g][(r & 31) * 4 + (r >> 5)] = scales;
+        for (int j = 0; j < 8; ++j) {
+            v[2 * j] = __uint_as_float(w[j] << 16);
+            v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
         }
-        if (sf_perm == nullptr) continue;
-        __syncthreads();   // (the other parity's buffer is written next: one barrier per unit is enough)
-        // the unit's atoms are contiguous: [row block][atom along K][512 bytes]
-        const int atoms_here = min(kQuantGroups, groups_per_row - unit_k * kQuantGroups);
-        const int atom = threadIdx.x >> 5, piece = threadIdx.x & 31;   // 16-byte piece of an atom
-        if (atom < atoms_here) {
-            uint8_t* dst = sf_perm + (static_cast<long long>(row_block) * groups_per_row + unit_k * kQuantGroups + atom) * 512 + piece * 16;
-            const uint32_t* st = &staged[parity][atom][piece * 4];
-            if (kWide) {
-                *reinterpret_cast<uint4*>(dst) = make_uint4(st[0], st[1], st[2], st[3]);
-            } else {
+    } else {
+        __half2 top = __habs2(*reinterpret_cast<const __half2*>(&w[0]));
 #pragma unroll
-                for (int b = 0; b < 16; ++b) dst[b] = static_cast<uint8_t>(st[b >> 2] >> (8 * (b & 3)));
-            }
+        for (int j = 1; j < 8; ++j) top = __hmax2_nan(top, __habs2(*reinterpret_cast<const __half2*>(&w[j])));
+        const float2 t = __half22float2(top);
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(amax) : "f"(t.x), "f"(t.y));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+            v[2 * j] = f.x;
+            v[2 * j + 1] = f.y;
+        }
+    }
+    return quantize_block16(v, amax, codes);
+}
+template <bool kWide>
+__device__ __forceinline__ void store_scale_word(uint8_t* at, uint32_t w) {
+    if (kWide) {
+        *reinterpret_cast<uint32_t*>(at) = w;
+    } else {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) at[b] = static_cast<uint8_t>(w >> (8 * b));
+    }
+}
+template <bool BF16, bool kWide, int R>
+__global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const QuantizeParams p) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int blocks = p.k / 16;
+    const unsigned col_units = (p.k + kQuantCols - 1) / kQuantCols;
+    const int unit_row = blockIdx.x / col_units;
+    const int row0 = unit_row * (8 * R) + warp * R;                                    // first row of this warp
+    const int blk = (blockIdx.x - unit_row * col_units) * (kQuantCols / 16) + lane;   // this lane's scale block
+    const bool in_row = blk < blocks;                                                  // (blocks is a multiple of four)
+    // A short quantiser stands between short GEMMs: its launch overlaps the end of the kernel before it.
+    ptx::grid_dependency_launch_dependents();
+    ptx::grid_dependency_wait();
+    const uint8_t* src = p.x + row0 * p.x_row_stride + blk * 32;
+    uint32_t w[R][8];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (in_row && row0 + r < p.rows) load_block16<kWide>(src + r * p.x_row_stride, w[r]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int row = row0 + r;
+        const bool exists = in_row && row < p.rows;
+        uint32_t scales = 0u;
+        if (exists) {
+            uint32_t codes[2];
+            scales = quantize_words<BF16>(w[r], codes) << (8 * (lane & 3));
+            *reinterpret_cast<uint2*>(p.packed + row * p.packed_row_stride + blk * 8) = make_uint2(codes[0], codes[1]);
+        }
+        scales |= __shfl_xor_sync(0xffffffffu, scales, 1);
+        scales |= __shfl_xor_sync(0xffffffffu, scales, 2);   // the scales of blocks blk & ~3 ... blk | 3
+        if (in_row && (lane & 3) == 0) {
+            if (p.sf_perm)   // rows of the last 128-row block that do not exist get zero scales
+                store_scale_word<kWide>(p.sf_perm + (static_cast<long long>(row / 128) * (blocks / 4) + blk / 4) * 512 + (row % 32) * 16 + (row % 128) / 32 * 4,
+                                        scales);
+            if (exists && p.sf_plain) store_scale_word<kWide>(p.sf_plain + row * p.sf_plain_row_stride + blk, scales);
         }
     }
 }

@@ -908,24 +908,43 @@ int nvfp4_quantize(const void* x, int32_t x_is_bf16, void* packed, void* sf_plai
     int dev = 0, sms = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // resident CTAs take 128-row x 256-column units in turn
-    const long long units = static_cast<long long>((rows + 127) / 128) * ((k / 64 + kQuantGroups - 1) / kQuantGroups);
-    const int grid = static_cast<int>(units < static_cast<long long>(sms) * 4 ? units : static_cast<long long>(sms) * 4);
-    // wide stores when every output address is aligned for them
-    const bool wide = aligned(packed, 16) && packed_row_stride % 16 == 0 && (!sf_plain || (aligned(sf_plain, 4) && sf_plain_row_stride % 4 == 0)) &&
+    QuantizeParams q;
+    q.x = static_cast<const uint8_t*>(x);
+    q.packed = static_cast<uint8_t*>(packed);
+    q.sf_plain = static_cast<uint8_t*>(sf_plain);
+    q.sf_perm = static_cast<uint8_t*>(sf_permuted);
+    q.rows = rows; q.k = k;
+    q.x_row_stride = 2 * x_row_stride; q.packed_row_stride = packed_row_stride; q.sf_plain_row_stride = sf_plain_row_stride;
+    // wide accesses when every address is aligned for them
+    const bool wide = aligned(x, 32) && x_row_stride % 16 == 0 && (!sf_plain || (aligned(sf_plain, 4) && sf_plain_row_stride % 4 == 0)) &&
                       (!sf_permuted || aligned(sf_permuted, 16));
-    auto launch = [&](auto kernel) {
-        kernel<<<grid, 256, 0, stream>>>(x, static_cast<uint8_t*>(packed), static_cast<uint8_t*>(sf_plain), static_cast<uint8_t*>(sf_permuted), rows, k,
-                                         x_row_stride, packed_row_stride, sf_plain_row_stride);
-    };
+    // (the permuted layout has scales for all rows of its last block; the plain one only for those that exist)
+    const long long out_rows = sf_permuted ? (rows + 127ll) / 128 * 128 : rows;
+    const long long col_units = (k + kQuantCols - 1) / kQuantCols;
+    auto units_of = [&](int rows_per_warp) { return (out_rows + 8 * rows_per_warp - 1) / (8 * rows_per_warp) * col_units; };
+    // Four rows per warp from 24 CTAs per SM on (between 4096 x 7168, 12 per SM, where one row is faster,
+    // and 8192 x 8192, 28 per SM, where four are: figures at the kernel).
+    const bool four = units_of(4) >= 24ll * sms;
+    const long long units = units_of(four ? 4 : 1);
+    if (units > 0x7fffffffll) return fail(NVFP4_ERR_INVALID_ARGUMENT, "problem too large: %lld work units", units);
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(static_cast<unsigned>(units), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto launch = [&](auto four_kernel, auto one_kernel) { return cudaLaunchKernelEx(&cfg, four ? four_kernel : one_kernel, q); };
     if (x_is_bf16) {
-        if (wide) launch(quantize_nvfp4_kernel<true, true>);
-        else launch(quantize_nvfp4_kernel<true, false>);
+        if (wide) CUDA_TRY(launch(quantize_nvfp4_kernel<true, true, 4>, quantize_nvfp4_kernel<true, true, 1>));
+        else CUDA_TRY(launch(quantize_nvfp4_kernel<true, false, 4>, quantize_nvfp4_kernel<true, false, 1>));
     } else {
-        if (wide) launch(quantize_nvfp4_kernel<false, true>);
-        else launch(quantize_nvfp4_kernel<false, false>);
+        if (wide) CUDA_TRY(launch(quantize_nvfp4_kernel<false, true, 4>, quantize_nvfp4_kernel<false, true, 1>));
+        else CUDA_TRY(launch(quantize_nvfp4_kernel<false, false, 4>, quantize_nvfp4_kernel<false, false, 1>));
     }
-    CUDA_TRY(cudaGetLastError());
     g_launches.fetch_add(1);
     return NVFP4_OK;
 }

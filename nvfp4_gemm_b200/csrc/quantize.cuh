@@ -7,6 +7,23 @@
 
 namespace nvfp4 {
 
+// Two fp32 values in one 64-bit register: sm_100 multiplies and adds them with one instruction.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+
 // One 16-element block -> eight bytes of e2m1 codes (out[0], out[1]; low nibble = lower index) and
 // the block's e4m3 scale byte: scale = RN-even saturating e4m3 of max|v| / 6, element =
 // RN-even saturating e2m1 of v / scale (all zero when the scale is zero).
@@ -17,20 +34,29 @@ namespace nvfp4 {
 // threshold that the true quotient hits, and everywhere else the quotient is at least 2^-11 away
 // (relatively) from a threshold because v has at most 11 significant bits and threshold * scale at
 // most 7.  Checked exhaustively on the CPU over every fp16 and bf16 value and every e4m3 scale.
-// Values beyond +-65504 (bf16 inputs, infinities) are clamped there first: the scale is then 448 and
-// the element saturates either way, while an infinity would poison the residual.
+// Values beyond +-65504 (bf16 inputs, infinities) are clamped there first, in a path of their own: the
+// scale is then 448 and the element saturates either way, while an infinity would poison the residual.
+//
+// What this costs in instructions is what the quantiser and the re-quantising epilogue are made of
+// besides their memory traffic, so the three multiplications and additions of an element are done two
+// elements at a time, and on -q instead of q (r negated): a residual of zero then carries the sign of
+// a zero through, which otherwise takes one more instruction per element, and the sign is turned
+// round for eight codes at once.
 // Eight bytes of e2m1 codes of v[0..15] / scale, scale > 0 an e4m3 value and |v| <= 65504.
 __device__ __forceinline__ void encode_block16(const float (&v)[16], float scale, uint32_t (&out)[2]) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(scale));
-    float q[16];
+    const uint64_t neg_r = pack_f32x2(-r, -r), scale2 = pack_f32x2(scale, scale);
+    float q[16];   // -(v / scale)
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const float a = v[j] * r;
-        q[j] = copysignf(fmaf(fmaf(-a, scale, v[j]), r, a), v[j]);   // the sign only differs for -0 (its residual is +0)
+    for (int j = 0; j < 8; ++j) {
+        const uint64_t x = pack_f32x2(v[2 * j], v[2 * j + 1]);
+        const uint64_t a = mul_f32x2(x, neg_r);
+        const uint64_t y = fma_f32x2(fma_f32x2(a, scale2, x), neg_r, a);
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(q[2 * j]), "=f"(q[2 * j + 1]) : "l"(y));
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h)   // four code bytes at a time (low nibble = lower index), packed by one move
+    for (int h = 0; h < 2; ++h) {  // four code bytes at a time (low nibble = lower index), packed by one move
         asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
             "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
             "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
@@ -40,12 +66,22 @@ __device__ __forceinline__ void encode_block16(const float (&v)[16], float scale
             : "=r"(out[h])
             : "f"(q[8 * h]), "f"(q[8 * h + 1]), "f"(q[8 * h + 2]), "f"(q[8 * h + 3]), "f"(q[8 * h + 4]), "f"(q[8 * h + 5]), "f"(q[8 * h + 6]),
               "f"(q[8 * h + 7]));
+        out[h] ^= 0x88888888u;
+    }
 }
 
-__device__ __forceinline__ uint8_t quantize_block16(const float (&v)[16], uint32_t (&out)[2]) {
-    float amax = 0.f;
+// amax: max|v|, NaN if any of v is one.  v is changed only where that or a value beyond 65504 occurs.
+__device__ __forceinline__ uint8_t quantize_block16(float (&v)[16], float amax, uint32_t (&out)[2]) {
+    if (!(amax <= 65504.f)) {
+        // A value beyond 65504, an infinity or a NaN, seldom enough to be sorted out here.  NaNs do not
+        // count towards the scale; one becomes +6 in a block that is otherwise within 65504, -6 in another.
+        amax = 0.f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[j]));
+        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[j]));
+        const float nan_as = amax <= 65504.f ? 65504.f : -65504.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = v[j] != v[j] ? nan_as : fminf(fmaxf(v[j], -65504.f), 65504.f);
+    }
     uint16_t sf_pair;
     // max|v| / 6 as a product with RN(1/6): the e4m3 rounding of the product equals that of the
     // exact quotient for every fp16 and bf16 value of max|v| (checked exhaustively on the CPU).
@@ -56,17 +92,15 @@ __device__ __forceinline__ uint8_t quantize_block16(const float (&v)[16], uint32
     const float scale = __low2float(*reinterpret_cast<__half2*>(&sf_h2));
     out[0] = 0u;
     out[1] = 0u;
-    if (scale > 0.f) {
-        if (amax <= 65504.f) {
-            encode_block16(v, scale, out);
-        } else {
-            float w[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) w[j] = fminf(fmaxf(v[j], -65504.f), 65504.f);
-            encode_block16(w, scale, out);
-        }
-    }
+    if (scale > 0.f) encode_block16(v, scale, out);
     return static_cast<uint8_t>(sf_pair & 0xff);
+}
+
+__device__ __forceinline__ uint8_t quantize_block16(float (&v)[16], uint32_t (&out)[2]) {
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) asm("max.NaN.f32 %0, %0, %1;" : "+f"(amax) : "f"(fabsf(v[j])));
+    return quantize_block16(v, amax, out);
 }
 
 }  // namespace nvfp4
