@@ -11,6 +11,7 @@
 #include <mutex>
 #include <string>
 
+#include "gemm_decode_sm100.cuh"
 #include "gemm_sm100.cuh"
 #include "gemv_sm100.cuh"
 #include "layout_kernels.cuh"
@@ -350,6 +351,37 @@ int launch_gemm_splitk(DeviceCtx* c, int variant, GemmParams& params, cudaStream
     return NVFP4_OK;
 }
 
+// Decode launch: one cluster of KS CTAs per 128 output columns.
+template <int BT, int STAGES, int KS>
+int launch_gemm_decode(const DeviceCtx* c, const GemmParams& params, bool epi, cudaStream_t stream, const char* name) {
+    using S = DecodeSmem<BT, STAGES, KS>;
+    auto kernel = epi ? gemm_decode_kernel<BT, STAGES, KS, true> : gemm_decode_kernel<BT, STAGES, KS, false>;
+    static std::atomic<uint64_t> attr_set[2];   // bit per device (ordinals are below 64)
+    if (!(attr_set[epi].load() >> c->device & 1u)) {
+        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamicBytes));
+        attr_set[epi].fetch_or(1ull << c->device);
+    }
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(params.tiles_n * params.L * KS, 1, 1);
+    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.dynamicSmemBytes = S::kDynamicBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = KS;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = KS > 1 ? 2 : 1;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, params));
+    g_launches.fetch_add(1);
+    t_last_kernel = name;
+    return NVFP4_OK;
+}
+
 __global__ void bounded_wait_selftest_kernel(int* status, unsigned long long timeout_cycles) {
     __shared__ uint64_t bar;
     __shared__ uint32_t abort_flag;
@@ -433,6 +465,58 @@ TileChoice choose_tile(int m, int n, int k, int l, int num_sms, const nvfp4_gemm
         if (cg == 1 && bn == 256 && (tiles256 < num_sms || (cf.cta_group == 0 && m > kBM))) bn = 128;
     }
     return TileChoice{cg, bn};
+}
+
+// The decode kernel (gemm_decode_sm100.cuh): how many tokens its tile holds and over how many CTAs K
+// is split.  split == 0: one of the other kernels.
+struct DecodeChoice {
+    int tokens, split;
+    bool two_per_sm;   // the shallow ring that lets two CTAs share an SM
+};
+// Rules measured on 17, 50 and 128 rows x 512 to 28672 columns x K 512 to 16384.  Splitting costs the
+// exchange (0.3-1 us) and pays when the k-tiles it takes off each CTA cost more:
+//   * 8 CTAs per tile only for up to eight tiles (clusters of eight do not fit side by side: 16 tiles run in
+//     two waves, 11.4 against 6.9 us) and K >= 12288 (17 x 512 x 16384: 5.05 us, four 5.94; x 7168: 4.03, 4.09);
+//   * 4 when they fit one wave: up to half a wave from K = 2048 (17 x 2048 x 2048: 3.31 us, unsplit 3.50),
+//     else from K = 6144 (17 x 4096 x 7168: 5.91, two 6.20; x 4096: 4.90, 4.92; 128 rows 6.77, 6.52);
+//   * 2 when they fit one wave: up to half a wave from K = 3072 (17 x 4096 x 4096: 4.92, unsplit
+//     5.33; x 2048: 3.89, 3.85), else from K = 6144 (17 x 7168 x 7168: 7.48, unsplit 7.87; x 4096: 5.79, 5.72).
+// More than 64 rows run here only when K is split (unsplit the 128-row-tile kernel is as fast or faster), so
+// two pays earlier: from K = 4096 on a whole wave (128 x 7168 x 4096: 7.38, 7.73 unsplit), and four from 3072.
+// More tiles than SMs: two CTAs per SM, so that one's start and end hide behind the other
+// (17 x 28672 x 2048: 7.07 against 9.29 us); up to one wave the deep ring is ahead (12288 columns: 4.55, 5.07).
+DecodeChoice choose_decode(int m, int n, int k, int l, int num_sms, const nvfp4_gemm_config& cf) {
+    if (m > kBM || cf.cta_group == 2 || cf.tile_n != 0 || cf.grid != 0 || cf.split_k != 0 || cf.epilogue != 0) return DecodeChoice{0, 0, false};
+    const int tokens = m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    const long long tiles = static_cast<long long>(n / kBM) * l;
+    const int k_tiles = k / kKPerStage;
+    const bool wide = tokens == 128;
+    int split = 1;
+    if (tiles <= 8 && k_tiles >= 48) split = 8;
+    else if (tiles * 4 <= num_sms && k_tiles >= (tiles * 8 <= num_sms ? (wide ? 12 : 8) : 24)) split = 4;
+    else if (tiles * 2 <= num_sms && k_tiles >= (tiles * 4 <= num_sms ? 12 : wide ? 16 : 24)) split = 2;
+    if (wide && split == 1) split = 0;
+    return DecodeChoice{tokens, split, split == 1 && tiles > num_sms};
+}
+
+int launch_gemm_decode(const DeviceCtx* c, const GemmParams& g, const DecodeChoice& d, bool epi, cudaStream_t stream) {
+    if (d.tokens == 32) {
+        if (d.split == 8) return launch_gemm_decode<32, 8, 8>(c, g, epi, stream, "gemm_splitk8_decode_t32");
+        if (d.split == 4) return launch_gemm_decode<32, 8, 4>(c, g, epi, stream, "gemm_splitk4_decode_t32");
+        if (d.split == 2) return launch_gemm_decode<32, 8, 2>(c, g, epi, stream, "gemm_splitk2_decode_t32");
+        if (d.two_per_sm) return launch_gemm_decode<32, 4, 1>(c, g, epi, stream, "gemm_decode_t32_s4");
+        return launch_gemm_decode<32, 8, 1>(c, g, epi, stream, "gemm_decode_t32_s8");
+    }
+    if (d.tokens == 64) {
+        if (d.split == 8) return launch_gemm_decode<64, 7, 8>(c, g, epi, stream, "gemm_splitk8_decode_t64");
+        if (d.split == 4) return launch_gemm_decode<64, 7, 4>(c, g, epi, stream, "gemm_splitk4_decode_t64");
+        if (d.split == 2) return launch_gemm_decode<64, 7, 2>(c, g, epi, stream, "gemm_splitk2_decode_t64");
+        if (d.two_per_sm) return launch_gemm_decode<64, 3, 1>(c, g, epi, stream, "gemm_decode_t64_s3");
+        return launch_gemm_decode<64, 7, 1>(c, g, epi, stream, "gemm_decode_t64_s7");
+    }
+    if (d.split == 8) return launch_gemm_decode<128, 4, 8>(c, g, epi, stream, "gemm_splitk8_decode_t128");
+    if (d.split == 4) return launch_gemm_decode<128, 4, 4>(c, g, epi, stream, "gemm_splitk4_decode_t128");
+    return launch_gemm_decode<128, 5, 2>(c, g, epi, stream, "gemm_splitk2_decode_t128");
 }
 
 int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_epilogue* epi, void* const* c_peers, int n_peers,
@@ -533,14 +617,6 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
     int epilogue = cf.epilogue;
     if (epilogue == 0) epilogue = 2;
     if (epi) epilogue = 1;                     // the extended epilogue writes with plain stores
-    if (epi && to_nvfp4 && g.out_sf_perm && p->m % 128) {
-        // rows of the last 128-row block that do not exist must read as zero scales
-        const long long last_block = static_cast<long long>((p->m + 127) / 128 - 1) * g.out_sf_perm_block_stride;
-        const long long tail = static_cast<long long>(p->n / 64) * 512;
-        for (int l = 0; l < p->l; ++l)
-            CUDA_TRY(cudaMemsetAsync(g.out_sf_perm + l * g.out_sf_perm_batch_stride + last_block, 0, tail, stream));
-    }
-
     const uint64_t kbytes = static_cast<uint64_t>(p->k) / 2;
     const uint64_t a_bs = p->l > 1 ? static_cast<uint64_t>(p->a_batch_stride) : static_cast<uint64_t>(p->a_row_stride) * p->m;
     const uint64_t b_bs = p->l > 1 ? static_cast<uint64_t>(p->b_batch_stride) : static_cast<uint64_t>(p->b_row_stride) * p->n;
@@ -566,20 +642,28 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
         }
     }
 
-    // Decode shapes (one 128-row block, fewer tiles than half the SMs): split K across a cluster
-    // and reduce through distributed shared memory instead of through global scratch.
-    int ks = cf.split_k;
-    if (ks == 0) {
-        ks = 1;
-        const long long tiles128 = static_cast<long long>(p->n / 128) * p->l;
-        if (p->m <= kBM && cf.cta_group != 2 && cf.tile_n == 0 && cf.grid == 0) {
-            // measured (four exchanges its partial sums through L2, two through distributed shared
-            // memory): four CTAs per tile win when they fit one wave (128 x 4096 x 7168: 10.1 vs
-            // 10.6 us), two otherwise (128 x 7168 x 16384: 17.5 us; 4 x 256-wide 20.3)
-            if (tiles128 * 4 <= c->num_sms && g.k_tiles >= 16 && !epi) ks = 4;
-            else if (tiles128 * 2 <= c->num_sms && g.k_tiles >= 16) ks = 2;   // shorter K: one whole tile per CTA wins
-        }
+    const DecodeChoice decode = choose_decode(p->m, p->n, p->k, p->l, c->num_sms, cf);
+    if (decode.split > 0 && n_peers == 0) {
+        g.tiles_m = 1;
+        g.tiles_n = p->n / kBM;
+        if (int rc = encode_map(make_key(p->a, kbytes, p->m, p->l, p->a_row_stride, a_bs, kBKBytes, decode.tokens, CU_TENSOR_MAP_DATA_TYPE_UINT8),
+                             &g.tma_a)) return rc;
+        if (int rc = encode_map(make_key(p->b, kbytes, p->n, p->l, p->b_row_stride, b_bs, kBKBytes, kBM, CU_TENSOR_MAP_DATA_TYPE_UINT8), &g.tma_b)) return rc;
+        if (int rc = encode_map(make_sf_key(p->sfb_perm, p->n, p->k, p->l, p->sfb_perm_batch_stride, 1), &g.tma_sfb)) return rc;
+        return launch_gemm_decode(c, g, decode, epi != nullptr, stream);
     }
+
+    if (epi && to_nvfp4 && g.out_sf_perm && p->m % 128) {
+        // rows of the last 128-row block that do not exist must read as zero scales (the decode kernel writes them itself)
+        const long long last_block = static_cast<long long>((p->m + 127) / 128 - 1) * g.out_sf_perm_block_stride;
+        const long long tail = static_cast<long long>(p->n / 64) * 512;
+        for (int l = 0; l < p->l; ++l)
+            CUDA_TRY(cudaMemsetAsync(g.out_sf_perm + l * g.out_sf_perm_batch_stride + last_block, 0, tail, stream));
+    }
+
+    // K split over a cluster of 128-row-tile CTAs, where the caller asks for it (decode shapes left to this
+    // library run the kernel above).
+    const int ks = cf.split_k ? cf.split_k : 1;
     if (ks > 1) {
         if (cf.cta_group == 2) return fail(NVFP4_ERR_INVALID_ARGUMENT, "split_k > 1 uses single-CTA tiles (cta_group 1)");
         if (g.k_tiles < ks) return fail(NVFP4_ERR_INVALID_ARGUMENT, "split_k = %d needs k >= %d", ks, ks * kKPerStage);
