@@ -1,7 +1,7 @@
 // NVFP4 block-scaled GEMV for sm_100a (CUDA cores; the op is HBM-bound, not a dense contraction):
 //   c[m, l] = sum_k  e2m1(a[m,k,l]) * sfa[m,k/16,l] * e2m1(b[k,l]) * sfb[k/16,l]
 //
-// One warp streams R rows; a lane owns 32-byte chunks (64 elements = 4 scale blocks) at a
+// gemv_nvfp4_kernel (K beyond 16384, or a launch shape the caller asks for): one warp streams R rows; a lane owns 32-byte chunks (64 elements = 4 scale blocks) at a
 // stride of 1024 bytes, so every warp-wide 256-bit load covers 1 KiB of contiguous row.  Per
 // 16-element block the products are summed in f16x2 (8 terms per half: exact), widened to fp32,
 // scaled by sfa*sfb and accumulated in fp32.  The vector and its scales are re-read through L1
@@ -184,6 +184,167 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_nvfp4_kernel(const GemvPara
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if (lane == 0 && row0 + r < p.M)
             p.c[l * p.c_batch_stride + static_cast<long long>(row0 + r) * p.c_row_stride] = __float2half_rn(v);
+    }
+}
+
+// The form for K up to 16384: the vector stays in registers.  A row worker is LANES lanes (or, for K
+// beyond 2048, k_warps whole warps side by side), a 64-element chunk of K per lane: it converts its
+// chunks of the vector once and walks rows of the matrix, four at a time with the next four in flight.
+// The matrix is then all that is loaded and converted, where the form above converts the vector again for
+// every R rows.  The partial sums of k_warps warps meet in shared memory.  The grid is resident at once
+// and the rows of all batches are split evenly over it, so short rows neither pay a CTA each nor end
+// in a ragged wave, and the launch can overlap the end of the kernel before it in the stream: the first
+// rows are asked into L2 ahead of the dependency wait.
+// Bound by HBM.  Measured (us, graph replay over rotating inputs, the form above -> this one): 7168 x 2048 x 4
+// 9.1 -> 7.6, 7168 x 16384 x 1 15.3 -> 13.2, 7168 x 16384 x 4 45.2 -> 43.9 (6.0 TB/s), 4096 x 7168 x 8
+// 26.3 -> 25.1; without the overlap of launches 8.9, 14.5, 45.6 and 26.4.
+constexpr int kGemvRowsPerStep = 4;
+constexpr int kGemvSliceChunks = 32;
+constexpr int kGemvMaxKWarps = 8;
+constexpr int kGemvBatchRows = 512;    // rows of a worker between two meetings of its warps
+
+// Sums of four values over LANES neighbouring lanes; lanes that are a multiple of LANES / 4 hold value
+// (lane % LANES) / (LANES / 4).
+template <int LANES>
+__device__ __forceinline__ float lanes_sum4(const float (&v)[4], int lane) {
+    const bool up = lane & (LANES / 2);
+    float a = up ? v[2] : v[0], b = up ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], LANES / 2);
+    b += __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], LANES / 2);
+    const bool up2 = lane & (LANES / 4);
+    float s = up2 ? b : a;
+    s += __shfl_xor_sync(0xffffffffu, up2 ? a : b, LANES / 4);
+#pragma unroll
+    for (int off = LANES / 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    return s;
+}
+
+template <int LANES>
+__global__ void __launch_bounds__(kGemvMaxKWarps * 32, 2) gemv_resident_kernel(const GemvParams p, int k_warps, int row_workers, int rows_each,
+                                                                               int rows_left) {
+    __shared__ float part[kGemvMaxKWarps * kGemvBatchRows];   // [row worker][row][k warp]
+    constexpr int R = kGemvRowsPerStep;
+    constexpr int kSub = 32 / LANES;                          // groups of lanes that take R rows each in a step of their warp
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int worker_in_cta = warp / k_warps, k_warp = warp % k_warps;
+    // rows [row_begin, row_end) of all batches' rows: rows_each per worker, the first rows_left workers take one more
+    const int worker = static_cast<int>(blockIdx.x) * row_workers + worker_in_cta;
+    const int row_begin = worker * rows_each + min(worker, rows_left), row_end = row_begin + rows_each + (worker < rows_left ? 1 : 0);
+    const int batch_rows = k_warps > 1 ? kGemvBatchRows : rows_each + 1;
+    const int batches = (rows_each + batch_rows) / batch_rows;   // the same for every warp of the grid
+    const int chunks = p.K / 64;
+    const int chunk_begin = k_warp * chunks / k_warps, chunk_end = (k_warp + 1) * chunks / k_warps;
+    const int chunk = chunk_begin + lane % LANES;
+    const int sub_row = lane / LANES * R;
+    const bool active = chunk < chunk_end;
+
+    // The first rows are asked into L2 ahead of the dependency wait (a prefetch consumes nothing).
+    if (active && row_begin < row_end) {
+        const int l = row_begin / p.M, row0 = row_begin - l * p.M;
+        const int n = min(min(sub_row + R, row_end - row_begin), p.M - row0);
+        const uint8_t* ptr = p.a + l * p.a_batch_stride + static_cast<long long>(row0) * p.a_row_stride + chunk * 32;
+        for (int r = sub_row; r < n; ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr + r * p.a_row_stride));
+    }
+    ptx::grid_dependency_launch_dependents();
+    ptx::grid_dependency_wait();
+
+    __half2 b2[32];
+    float sfb[4];
+    int loaded_l = -1;
+    for (int batch = 0; batch < batches; ++batch) {
+        const int batch_begin = min(row_begin + batch * batch_rows, row_end);
+        const int batch_end = min(batch_begin + batch_rows, row_end);
+        for (int seg = batch_begin; seg < batch_end;) {   // rows of one l
+            const int l = seg / p.M;
+            const int row0 = seg - l * p.M;
+            const int n_rows = min(batch_end - seg, p.M - row0);
+            const uint8_t* a_ptr = p.a + l * p.a_batch_stride + static_cast<long long>(row0 + sub_row) * p.a_row_stride + chunk * 32;
+            const uint8_t* sfa_ptr = p.sfa + l * p.sfa_batch_stride + static_cast<long long>(row0 + sub_row) * p.sfa_row_stride + chunk * 4;
+            Chunk32 next[R];
+            uint32_t next_sf[R];
+            auto fetch = [&](int row) {   // rows [row + sub_row, + R) of the segment; the pointers stand at the first
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (active && row + sub_row + r < n_rows) {
+                        next[r] = ld_stream_32B(a_ptr);
+                        next_sf[r] = ld_stream_u32(sfa_ptr);
+                    }
+                    a_ptr += p.a_row_stride;
+                    sfa_ptr += p.sfa_row_stride;
+                }
+                if constexpr (kSub > 1) {
+                    a_ptr += (kSub - 1) * R * p.a_row_stride;
+                    sfa_ptr += (kSub - 1) * R * p.sfa_row_stride;
+                }
+            };
+#pragma unroll
+            for (int r = 0; r < R; ++r) { next[r] = Chunk32{}; next_sf[r] = 0u; }
+            fetch(0);
+            if (l != loaded_l) {
+                loaded_l = l;
+                Chunk32 bv{};
+                uint32_t sbv = 0u;
+                if (active) {
+                    bv = ld_keep_32B(p.b + l * p.b_batch_stride + chunk * 32);
+                    sbv = ld_keep_u32(p.sfb + l * p.sfb_batch_stride + chunk * 4);
+                }
+                cvt_e4m3x4(sbv, sfb);
+#pragma unroll
+                for (int w = 0; w < 8; ++w) {
+                    uint32_t t[4];
+                    cvt_e2m1x8(bv.w[w], t);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) b2[4 * w + e] = *reinterpret_cast<__half2*>(&t[e]);
+                }
+            }
+            for (int row = 0; row < n_rows; row += R * kSub) {
+                Chunk32 cur[R];
+                uint32_t cur_sf[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) { cur[r] = next[r]; cur_sf[r] = next_sf[r]; }
+                fetch(row + R * kSub);
+                float sum[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    float sfa[4];
+                    cvt_e4m3x4(cur_sf[r], sfa);
+                    sum[r] = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {   // one scale block: eight exact products per half, then fp32
+                        uint32_t t0[4], t1[4];
+                        cvt_e2m1x8(cur[r].w[2 * j], t0);
+                        cvt_e2m1x8(cur[r].w[2 * j + 1], t1);
+                        __half2 acc = __float2half2_rn(0.f);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc = __hfma2(*reinterpret_cast<__half2*>(&t0[e]), b2[8 * j + e], acc);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc = __hfma2(*reinterpret_cast<__half2*>(&t1[e]), b2[8 * j + 4 + e], acc);
+                        const float2 s = __half22float2(acc);
+                        sum[r] = fmaf(s.x + s.y, sfa[j] * sfb[j], sum[r]);
+                    }
+                    if (!active) sum[r] = 0.f;      // (lanes past the slice: whatever they hold does not count)
+                }
+                const float s = lanes_sum4<LANES>(sum, lane);
+                const int r = sub_row + lane % LANES / (LANES / 4);
+                if (lane % (LANES / 4) == 0 && row + r < n_rows) {
+                    if (k_warps == 1) p.c[l * p.c_batch_stride + static_cast<long long>(row0 + row + r) * p.c_row_stride] = __float2half_rn(s);
+                    else part[(worker_in_cta * kGemvBatchRows + seg - batch_begin + row + r) * k_warps + k_warp] = s;
+                }
+            }
+            seg += n_rows;
+        }
+        if (k_warps > 1) {
+            __syncthreads();
+            for (int i = k_warp * 32 + lane; i < batch_end - batch_begin; i += k_warps * 32) {
+                const float* src = part + (worker_in_cta * kGemvBatchRows + i) * k_warps;
+                float v = 0.f;
+                for (int w = 0; w < k_warps; ++w) v += src[w];
+                const int row = batch_begin + i;
+                const int l = row / p.M;
+                p.c[l * p.c_batch_stride + static_cast<long long>(row - l * p.M) * p.c_row_stride] = __float2half_rn(v);
+            }
+            __syncthreads();
+        }
     }
 }
 

@@ -779,6 +779,40 @@ int nvfp4_gemv_config(const nvfp4_problem* p, int rows_per_warp, int warps_per_c
     if (int rc = gemv_prepare(p, &g)) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 
+    // Up to K = 16384 the vector fits the registers of the warps that share a row.  Lanes per row: as many
+    // as it has 64-element chunks, rounded up to 8, 16 or 32 (more lanes would idle: 28672 x 512 x 8 took 48.4 us
+    // with a warp per row and 15.3 with 8 lanes), and no more CTAs than have a whole step of rows to do
+    // (2000 x 1024 x 8: 4.8 -> 3.7 us).
+    const long long rows_total = static_cast<long long>(p->m) * p->l;
+    const int chunks = p->k / 64;
+    if (rows_per_warp == 0 && warps_per_cta == 0 && chunks <= kGemvMaxKWarps * kGemvSliceChunks && rows_total < (1 << 30)) {
+        DeviceCtx* c = nullptr;
+        if (int rc = get_ctx(&c)) return rc;
+        const int k_warps = (chunks + kGemvSliceChunks - 1) / kGemvSliceChunks;
+        const int row_workers = kGemvMaxKWarps / k_warps;
+        const int lanes = chunks <= 8 ? 8 : chunks <= 16 ? 16 : 32;
+        const long long step_rows = static_cast<long long>(row_workers) * kGemvRowsPerStep * (32 / lanes);   // one step of a CTA
+        long long ctas = (rows_total + step_rows - 1) / step_rows;
+        if (ctas > 2LL * c->num_sms) ctas = 2LL * c->num_sms;      // two fit an SM (128 registers x 256 threads)
+        cudaLaunchConfig_t cfg;
+        std::memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+        cfg.blockDim = dim3(k_warps * row_workers * 32, 1, 1);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        auto kernel = lanes == 8 ? gemv_resident_kernel<8> : lanes == 16 ? gemv_resident_kernel<16> : gemv_resident_kernel<32>;
+        const long long workers = ctas * row_workers;
+        CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, g, k_warps, row_workers, static_cast<int>(rows_total / workers),
+                                    static_cast<int>(rows_total % workers)));
+        g_launches.fetch_add(1);
+        t_last_kernel = lanes == 8 ? "gemv_resident_8" : lanes == 16 ? "gemv_resident_16" : "gemv_resident_32";
+        return NVFP4_OK;
+    }
+
     // Rows per warp: short rows amortise the vector's dequantisation over four rows; long rows keep
     // more loads in flight with two, or with one when there are so few rows that two per warp
     // would leave warps short.  One warp per CTA: the block scheduler hands out CTAs as SMs free
@@ -788,13 +822,11 @@ int nvfp4_gemv_config(const nvfp4_problem* p, int rows_per_warp, int warps_per_c
     // r4/w1 9.1, r2 10.1, r1 14.4.  (Splitting K over the warps of a CTA, one CTA per one or two
     // rows, was measured as well: 14.7 us at best on 7168 x 16384 x 1 and slower than this
     // everywhere else, so it is not kept.)
-    const long long rows_total = static_cast<long long>(p->m) * p->l;
     const int r = rows_per_warp ? rows_per_warp : (p->k <= 4096) ? 4 : (rows_total <= 8192) ? 1 : 2;
     const int w = warps_per_cta ? warps_per_cta : 1;
     const int rows_per_cta = w * r;
     dim3 grid((p->m + rows_per_cta - 1) / rows_per_cta, p->l);
-    // (Programmatic dependent launch, which the GEMM kernels use, was measured here too: no gain on
-    // the long shapes and 9.0 -> 9.9 us on 7168 x 2048 x 4, so the GEMV is launched plainly.)
+    // (Programmatic dependent launch gained nothing with these one-warp CTAs.)
     if (r == 4) gemv_nvfp4_kernel<4><<<grid, w * 32, 0, stream>>>(g);
     else if (r == 2) gemv_nvfp4_kernel<2><<<grid, w * 32, 0, stream>>>(g);
     else gemv_nvfp4_kernel<1><<<grid, w * 32, 0, stream>>>(g);

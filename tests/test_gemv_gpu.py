@@ -44,6 +44,46 @@ def test_gemv_benchmark_shapes(sub, oracle, shape):
     assert_bit_exact(out, expected_fp16(oracle, data), what=f"gemv {shape}")
 
 
+# edges of the kernel that keeps the vector in registers: 8, 16 and 32 lanes per row full and just beyond,
+# one to eight warps per row with even and uneven slices, fewer rows than workers, rows of several
+# batches in one worker, more rows than workers' warps meet over at once; and the first K beyond it
+@pytest.mark.parametrize("shape", [(1, 512, 1), (3, 448, 5), (5000, 512, 2), (1025, 576, 3), (40, 1024, 9), (2400, 1088, 1), (77, 2048, 4), (3001, 2112, 2),
+                                   (2, 4096, 3), (601, 6208, 2), (1000, 10304, 1), (5, 16384, 7), (297, 16384, 1), (40000, 2112, 4), (9, 16448, 2)])
+def test_gemv_resident_edges(sub, oracle, shape):
+    from nvfp4_gemm_b200.inputs import generate_input
+    m, k, l = shape
+    data = generate_input(m, 1, k, l, 12)
+    exp = expected_fp16(oracle, data)
+    for _ in range(2):
+        data[6].view(torch.int16).fill_(0x7fff)
+        sub.custom_kernel(data)
+        torch.cuda.synchronize()
+        assert sub.last_kernel().startswith("gemv_resident" if k <= 16384 else "gemv_warp")
+        assert_bit_exact(data[6], exp, what=f"gemv {shape}")
+
+
+def test_gemv_back_to_back_launches_respect_stream_order(sub, lib):
+    """The matrix-vector product may start before the kernel ahead of it has ended; its operands are
+    rewritten in place right before each launch."""
+    from nvfp4_gemm_b200.inputs import generate_input
+    sets = [generate_input(2048, 1, 4096, 1, s) for s in (1, 2, 3)]
+    exp = []
+    for d in sets:
+        sub.custom_kernel(d)
+        torch.cuda.synchronize()
+        exp.append(d[6].clone())
+    work = [t.clone(memory_format=torch.preserve_format) for t in sets[0]]
+    outs = []
+    for _ in range(5):
+        for d in sets:
+            for i in range(4):
+                work[i].view(torch.uint8).copy_(d[i].view(torch.uint8))
+            outs.append(sub.custom_kernel(tuple(work)).clone())
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        assert torch.equal(o.view(torch.int16), exp[i % 3].view(torch.int16)), i
+
+
 def test_gemv_general_scales_within_tolerance(sub, oracle):
     from nvfp4_gemm_b200.inputs import generate_input, SF_DTYPE
     m, k, l = 256, 4096, 2
