@@ -34,6 +34,8 @@
 
 namespace nvfp4 {
 
+constexpr int kDecodeThreads = 192;
+
 template <int BT, int STAGES, int KS>
 struct DecodeSmem {
     static constexpr uint32_t kWBytes = kBM * kBKBytes;               // weights: 128 rows of 256 e2m1
@@ -84,7 +86,7 @@ __device__ __forceinline__ void bias_act16(const GemmParams& p, int gcol, float*
 constexpr int kDecodeSfwCol = 128, kDecodeSfxCol = 160, kDecodeTmemCols = 256;
 
 template <int BT, int STAGES, int KS, bool EPI_EX>
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __grid_constant__ GemmParams p) {
     using S = DecodeSmem<BT, STAGES, KS>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_decode_kernel(const __gr
     ptx::grid_dependency_launch_dependents();
     ptx::grid_dependency_wait();
     if (warp != 0) {
-        ptx::named_bar_sync(3, kGemmThreads - 32);
+        ptx::named_bar_sync(3, kDecodeThreads - 32);
         ptx::tc_fence_after();
         tmem_base = *tmem_slot_gen;
     }

@@ -13,7 +13,7 @@
 // (CG = 2: 256 x BN tile; each CTA holds 128 rows of A, BN/2 rows of B and its own 128
 // accumulator rows, so B crosses L2 -> SM once per pair).
 //
-// Warp roles (192 threads per CTA):
+// Warp roles (320 threads per CTA; 192 in the cluster split-K kernels):
 //   warp 0      TMA producer: A/B tiles (128-byte swizzle) and the 512-byte scale atoms of the
 //               permuted layout into a STAGES-deep shared-memory ring (full/empty mbarriers)
 //   warp 1      TMEM owner.  Leader CTA: MMA issuer, ONE thread elected once -- tcgen05.cp scale
@@ -21,7 +21,7 @@
 //               stage, tcgen05.commit to release the stage / publish the accumulator.  In a pair
 //               both CTAs' loads signal the leader's full barrier (cp.async.bulk.tensor
 //               .cta_group::2).
-//   warps 2..5  epilogue: tcgen05.ld -> fp16 -> TMA store (or 16-byte stores), or the fp32
+//   warps 2..9  (2..5) epilogue: tcgen05.ld -> fp16 -> TMA store (or 16-byte stores), or the fp32
 //               partial-tile path
 //
 // No load in this file uses cluster multicast; the only cluster-wide signals are mbarrier
@@ -40,7 +40,6 @@ constexpr int kBKBytes = 128;      // bytes of K per stage row = one 128-byte sw
 constexpr int kKPerStage = 256;    // K elements per stage
 constexpr int kMmaPerStage = 4;    // K = 64 per tcgen05.mma
 constexpr int kSfAtomBytes = 512;  // 128 rows x 4 scales
-constexpr int kGemmThreads = 192;
 constexpr int kTmemCols = 512;
 // TMEM columns.  128-wide tiles: two accumulators [0,128) and [128,256), scale buffers behind
 // them.  256-wide tiles of the persistent kernels: two accumulators that OVERLAP by half,
@@ -115,7 +114,11 @@ struct GemmSmem {
     // Epilogue scratch: TMA-store staging (two 32-row x 128-byte buffers per warp), or the landing
     // area of the cluster split-K exchange.
     static constexpr uint32_t kEpiBytes = EPI_KB * 1024;
-    static constexpr uint32_t kStagingBufs = TMA_STORE ? (EPI_KB * 1024 / 4) / 4096 : 2;   // 32-row x 128-byte buffers per epilogue warp
+    // Epilogue warps: two groups of four (each covers the 128 TMEM lanes) share a tile's columns; the
+    // cluster split-K kernels have one group.
+    static constexpr int kEpiWarps = KS == 1 ? 8 : 4;
+    static constexpr int kThreads = 64 + 32 * kEpiWarps;
+    static constexpr uint32_t kStagingBufs = TMA_STORE ? (EPI_KB * 1024 / kEpiWarps) / 4096 : 1;   // 32-row x 128-byte buffers per epilogue warp
     static constexpr uint32_t kStagingPerWarp = kStagingBufs * 32 * 128;
     static constexpr uint32_t kFixBufs = 2;   // barriers of the cluster split-K exchange ("landed", "ready")
     static constexpr uint32_t kEpiOff = STAGES * kStageBytes;
@@ -135,7 +138,7 @@ struct GemmSmem {
     static constexpr uint32_t kBytes = kBarOff + kNumBars * 8 + 16;
     static constexpr uint32_t kDynamicBytes = kBytes + 1024;  // slack for manual 1024-byte alignment
     static_assert(kStageBytes % 1024 == 0, "stage tiles must keep 1024-byte alignment");
-    static_assert(!TMA_STORE || kEpiBytes >= 4 * kStagingPerWarp, "TMA-store staging does not fit");
+    static_assert(!TMA_STORE || (kStagingBufs >= 1 && kEpiBytes >= kEpiWarps * kStagingPerWarp), "TMA-store staging does not fit");
     static_assert(KS == 1 || (CG == 1 && BN / KS >= 32 && STAGES * kStageBytes >= kBM * BN * 4),
                   "cluster split-K: single-CTA MMAs, at least 32 columns per CTA, the ring must hold one fp32 tile");
     static_assert(kDynamicBytes <= 232448, "exceeds the 227 KB of shared memory one CTA may use");
@@ -247,7 +250,7 @@ __device__ __forceinline__ uint4 pack8_fp16(const uint32_t* v) {
 }
 
 template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1, bool EPI_EX = false>
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS>::kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ GemmParams p) {
     static_assert(!(EPI_EX && TMA_STORE), "the extended epilogue writes with plain stores");
     using S = GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS>;
     constexpr int kNumAcc = S::kNumAcc;
@@ -258,6 +261,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
     // An overlapped accumulator is drained shared half first and released once that half is in
     // registers; a plain one after its last column.
     constexpr int kReleaseAfter = kAccOverlap ? kChunks / 2 : kChunks;
+    constexpr int kEpiThreads = 32 * S::kEpiWarps;
+    constexpr int kGroups = S::kEpiWarps / 4;                          // epilogue warp groups
+    constexpr int kMyRelease = kReleaseAfter / kGroups;                // pieces a group drains before the hand-back
+    constexpr int kMyChunks = kChunks / kGroups;                       // pieces a group drains in all
     constexpr int kSfbColsPerMma = BN / 32;  // 4 TMEM columns per 128 rows of B
     constexpr int kBRows = S::kBRows;
 
@@ -294,7 +301,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
             ptx::mbar_init(bar_fix_full + b * 8, (KS > 1 && b == 0) ? (S::kBulkExchange ? 1 : 128 * (KS - 1)) : (KS > 1 && b == 1) ? (KS - 1) : 1);
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(bar_acc_full + a * 8, 1);
-            ptx::mbar_init(bar_acc_empty + a * 8, 128 * CG);
+            ptx::mbar_init(bar_acc_empty + a * 8, kEpiThreads * CG);
         }
         *abort_flag = 0u;
         ptx::fence_mbar_init();
@@ -369,7 +376,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
     ptx::grid_dependency_launch_dependents();
     ptx::grid_dependency_wait();
     if (warp != 0) {
-        ptx::named_bar_sync(3, kGemmThreads - 32);
+        ptx::named_bar_sync(3, S::kThreads - 32);
         ptx::tc_fence_after();
         tmem_base = *tmem_slot_gen;
     }
@@ -522,7 +529,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
         // ------------------------------------------------------------ epilogue
         const int quad = warp & 3;             // TMEM lane quadrant this warp may read
         const int row_in_tile = quad * 32 + lane;
-        const int epi_tid = threadIdx.x - 64;  // 0..127
+        const int epi_tid = threadIdx.x - 64;
+        const int group = (warp - 2) / 4;      // which share of a tile's columns
         uint32_t acc_it = 0;
         uint32_t store_buf = 0;
         // NVFP4 output: whether 32-byte code stores and 4-byte scale stores are aligned
@@ -541,19 +549,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
             const int l = tc.l;
             const uint32_t acc = acc_it % kNumAcc;
             const uint32_t acc_phase = (acc_it / kNumAcc) & 1u;
-            // All 128 epilogue threads take the same branch: the outcome of the wait is agreed on
+            // All epilogue threads take the same branch: the outcome of the wait is agreed on
             // through a barrier, so a thread that gave up cannot strand the others at a later one.
             bool got_acc;
             {
                 got_acc = ptx::mbar_wait_bounded(bar_acc_full + acc * 8, acc_phase, abort_flag, timeout);
             }
-            if (!ptx::named_bar_and(2, 128, got_acc)) break;
+            if (!ptx::named_bar_and(2, kEpiThreads, got_acc)) break;
             ptx::tc_fence_after();
             const uint32_t t_acc = tmem_base + acc * S::kAccStride + (static_cast<uint32_t>(quad * 32) << 16);
             // drain order: position p reads chunk (p + first_chunk) mod kChunks, so that the half an
             // overlapped accumulator shares with the other one comes first
             const int first_chunk = (kAccOverlap && acc == 0) ? kChunks / 2 : 0;
             auto chunk_at = [&](int pos) { return (pos + first_chunk) & (kChunks - 1); };
+            // the i-th piece this group drains: its share of those ahead of the hand-back, then of the others
+            auto my_chunk = [&](int i) {
+                return chunk_at(i < kMyRelease ? group * kMyRelease + i : kReleaseAfter + group * (kMyChunks - kMyRelease) + (i - kMyRelease));
+            };
             const bool whole_tile = (k1 - k0 == KT);
             const int row = mb * kBM + row_in_tile;
             const long long c_off = l * p.c_batch_stride + static_cast<long long>(row) * p.c_row_stride + nb * BN;
@@ -819,20 +831,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                     // 64 columns (128 bytes of fp16) at a time through a swizzled 32-row staging buffer.
                     uint8_t* staging_gen = smem_gen + S::kEpiOff + (warp - 2) * S::kStagingPerWarp;
                     const uint32_t staging = smem_base + S::kEpiOff + (warp - 2) * S::kStagingPerWarp;
-                    // Phase 1, drain: the whole accumulator row of this thread goes TMEM -> registers
-                    // -> fp16 pairs (BN/2 registers), the loads of the next 32 columns in flight while
+                    // Phase 1, drain: this thread's share of its accumulator row goes TMEM -> registers
+                    // -> fp16 pairs (BN/4 registers), the loads of the next 32 columns in flight while
                     // the previous ones are converted.  The accumulator is handed back to the MMA warp
                     // as soon as the last column is in registers, before anything is stored: the TMA
                     // stores queue behind the producer's loads in the same TMA unit and are slow to
                     // free their staging buffer.
-                    uint32_t packed[BN / 2];          // by drain position
+                    uint32_t packed[kMyChunks * 16];
                     uint32_t v[2][32];
-                    ptx::tc_ld_32cols(t_acc + chunk_at(0) * 32, v[0]);
+                    ptx::tc_ld_32cols(t_acc + my_chunk(0) * 32, v[0]);
 #pragma unroll
-                    for (int pos = 0; pos < kChunks; ++pos) {
+                    for (int pos = 0; pos < kMyChunks; ++pos) {
                         ptx::tc_wait_ld();
-                        if (pos + 1 < kChunks) ptx::tc_ld_32cols(t_acc + chunk_at(pos + 1) * 32, v[(pos + 1) & 1]);
-                        if (pos + 1 == kReleaseAfter) release_acc();
+                        if (pos + 1 < kMyChunks) ptx::tc_ld_32cols(t_acc + my_chunk(pos + 1) * 32, v[(pos + 1) & 1]);
+                        if (pos + 1 == kMyRelease) release_acc();
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             const __half2 h = __floats2half2_rn(__uint_as_float(v[pos & 1][2 * j]), __uint_as_float(v[pos & 1][2 * j + 1]));
@@ -842,7 +854,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                     // Phase 2, store: 64 columns (128 bytes of fp16) at a time through the swizzled
                     // 32-row staging buffers, overlapping the next tile's MMAs.
 #pragma unroll
-                    for (int ci = 0; ci < BN / 64; ++ci) {
+                    for (int ci = 0; ci < kMyChunks / 2; ++ci) {
                         // the buffer about to be overwritten was read by the store issued kStagingBufs chunks ago
                         if (lane == 0) ptx::bulk_wait_group_read<S::kStagingBufs - 1>();
                         __syncwarp();
@@ -854,10 +866,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                         ptx::fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0 && mb * kBM + quad * 32 < p.M) {  // rows past M inside the box are clipped; one fixed lane owns the bulk groups
-                            ptx::tma_store_3d(&p.tma_c, staging + store_buf * 4096, nb * BN + chunk_at(2 * ci) * 32, mb * kBM + quad * 32, l);
+                            ptx::tma_store_3d(&p.tma_c, staging + store_buf * 4096, nb * BN + my_chunk(2 * ci) * 32, mb * kBM + quad * 32, l);
                             if (p.peer_tma)   // the same block to every peer, in the same bulk group: the buffer is free when all have read it
                                 for (int r = 0; r < p.n_peer; ++r)
-                                    ptx::tma_store_3d(&p.tma_c_peer[r], staging + store_buf * 4096, nb * BN + chunk_at(2 * ci) * 32, mb * kBM + quad * 32, l);
+                                    ptx::tma_store_3d(&p.tma_c_peer[r], staging + store_buf * 4096, nb * BN + my_chunk(2 * ci) * 32, mb * kBM + quad * 32, l);
                             ptx::bulk_commit_group();
                         }
                         if (p.n_peer > 0 && !p.peer_tma) {
@@ -875,7 +887,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                             const int row_base = mb * kBM + quad * 32;
                             for (int pi = 0; pi < p.n_peer; ++pi) {
                                 const int r = (pi + static_cast<int>(blockIdx.x)) % p.n_peer;   // spread the start over CTAs
-                                __half* dst = p.c_peer[r] + l * p.c_batch_stride + nb * BN + chunk_at(2 * ci) * 32 + piece * 8;
+                                __half* dst = p.c_peer[r] + l * p.c_batch_stride + nb * BN + my_chunk(2 * ci) * 32 + piece * 8;
 #pragma unroll
                                 for (int it = 0; it < 8; ++it) {
                                     const int grow = row_base + it * 4 + sub;
@@ -909,17 +921,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                                                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
                     };
                     if constexpr (kAccOverlap) {
-                        uint32_t held[kReleaseAfter][32];
+                        uint32_t held[kMyRelease][32];
 #pragma unroll
-                        for (int pos = 0; pos < kReleaseAfter; ++pos) ptx::tc_ld_32cols(t_acc + chunk_at(pos) * 32, held[pos]);
+                        for (int pos = 0; pos < kMyRelease; ++pos) ptx::tc_ld_32cols(t_acc + my_chunk(pos) * 32, held[pos]);
                         ptx::tc_wait_ld();
                         release_acc();  // the MMA warp may start the next tile now
 #pragma unroll
-                        for (int pos = 0; pos < kReleaseAfter; ++pos) publish32(chunk_at(pos) * 32, held[pos]);
+                        for (int pos = 0; pos < kMyRelease; ++pos) publish32(my_chunk(pos) * 32, held[pos]);
                     }
 #pragma unroll 1
-                    for (int pos = kAccOverlap ? kReleaseAfter : 0; pos < kChunks; ++pos) {
-                        const int c0 = chunk_at(pos) * 32;
+                    for (int pos = kAccOverlap ? kMyRelease : 0; pos < kMyChunks; ++pos) {
+                        const int c0 = my_chunk(pos) * 32;
                         uint32_t v[32];
                         ptx::tc_ld_32cols(t_acc + c0, v);
                         ptx::tc_wait_ld();
@@ -927,7 +939,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                     }
                     if constexpr (!kAccOverlap) release_acc();
                     __threadfence();
-                    ptx::named_bar_sync(1, 128);
+                    ptx::named_bar_sync(1, kEpiThreads);
                     if (epi_tid == 0) atomicAdd(counter, k1 - k0);
                 } else {
                     // Finish: the rest of the k-range has been published (normally long ago); add
@@ -938,12 +950,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                     const int w_last = whole_tile ? w_first : unit_owner(tile * KT + KT - 1, n_workers, p.total_units);
                     const int need = KT - (k1 - k0);
                     // Everything the hand-back waits for goes to registers first (the half an
-                    // overlapped accumulator shares with the other one, else all of it: at most four
-                    // 32-column pieces), the accumulator is released, and only then anything is
+                    // overlapped accumulator shares with the other one, else all of it: two
+                    // 32-column pieces per thread), the accumulator is released, and only then anything is
                     // waited for, converted or stored.
-                    uint32_t held[kReleaseAfter][32];
+                    uint32_t held[kMyRelease][32];
 #pragma unroll
-                    for (int pos = 0; pos < kReleaseAfter; ++pos) ptx::tc_ld_32cols(t_acc + chunk_at(pos) * 32, held[pos]);
+                    for (int pos = 0; pos < kMyRelease; ++pos) ptx::tc_ld_32cols(t_acc + my_chunk(pos) * 32, held[pos]);
                     ptx::tc_wait_ld();
                     release_acc();
                     if (!whole_tile) {
@@ -959,9 +971,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                                 __nanosleep(64);
                             }
                         }
-                        if (!ptx::named_bar_and(1, 128, ready)) break;
+                        if (!ptx::named_bar_and(1, kEpiThreads, ready)) break;
                     }
-                    static_assert(kChunks % 2 == 0 && kReleaseAfter % 2 == 0, "the partial sums are added 64 columns at a time");
+                    static_assert(kMyChunks % 2 == 0 && kMyRelease % 2 == 0, "the partial sums are added 64 columns at a time");
                     // the columns [c0a, c0a + 32) and [c0b, c0b + 32) of this thread's row: own sums in, total out
                     auto add_others_and_emit = [&](int c0a, int c0b, float (&sa)[32], float (&sb)[32]) {
 #pragma unroll 1
@@ -981,22 +993,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_nvfp4_kernel(const __gri
                         if (row < p.M) emit64(c0a, sa, sb);   // (c0b == c0a + 32: drain positions pair up neighbouring chunks)
                     };
 #pragma unroll
-                    for (int pos = 0; pos < kReleaseAfter; pos += 2) {
+                    for (int pos = 0; pos < kMyRelease; pos += 2) {
                         float sa[32], sb[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) { sa[i] = __uint_as_float(held[pos][i]); sb[i] = __uint_as_float(held[pos + 1][i]); }
-                        add_others_and_emit(chunk_at(pos) * 32, chunk_at(pos + 1) * 32, sa, sb);
+                        add_others_and_emit(my_chunk(pos) * 32, my_chunk(pos + 1) * 32, sa, sb);
                     }
 #pragma unroll 1
-                    for (int pos = kReleaseAfter; pos < kChunks; pos += 2) {
+                    for (int pos = kMyRelease; pos < kMyChunks; pos += 2) {
                         uint32_t va[32], vb[32];
-                        ptx::tc_ld_32cols(t_acc + chunk_at(pos) * 32, va);
-                        ptx::tc_ld_32cols(t_acc + chunk_at(pos + 1) * 32, vb);
+                        ptx::tc_ld_32cols(t_acc + my_chunk(pos) * 32, va);
+                        ptx::tc_ld_32cols(t_acc + my_chunk(pos + 1) * 32, vb);
                         ptx::tc_wait_ld();
                         float sa[32], sb[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) { sa[i] = __uint_as_float(va[i]); sb[i] = __uint_as_float(vb[i]); }
-                        add_others_and_emit(chunk_at(pos) * 32, chunk_at(pos + 1) * 32, sa, sb);
+                        add_others_and_emit(my_chunk(pos) * 32, my_chunk(pos + 1) * 32, sa, sb);
                     }
                     if (!whole_tile && epi_tid == 0) *counter = 0;
                 }

@@ -266,7 +266,7 @@ int launch_gemm(DeviceCtx* c, int variant, GemmParams& params, int grid_request,
     }
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.blockDim = dim3(S::kThreads, 1, 1);
     cfg.dynamicSmemBytes = S::kDynamicBytes;
     cfg.stream = stream;
     // programmatic dependent launch: the kernel's set-up may overlap the tail of the kernel before
@@ -326,7 +326,7 @@ int launch_gemm_splitk(DeviceCtx* c, int variant, GemmParams& params, cudaStream
     }
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.blockDim = dim3(S::kThreads, 1, 1);
     cfg.dynamicSmemBytes = S::kDynamicBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -364,7 +364,7 @@ int launch_gemm_decode(const DeviceCtx* c, const GemmParams& params, bool epi, c
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(params.tiles_n * params.L * KS, 1, 1);
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.blockDim = dim3(kDecodeThreads, 1, 1);
     cfg.dynamicSmemBytes = S::kDynamicBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -1315,7 +1315,7 @@ int nvfp4_gemm_static_scratch(const nvfp4_problem* p, int workers, void* stream_
     // are read, but the per-tile counters must start at zero (an aborted launch may have left some).
     CUDA_TRY(cudaMemsetAsync(st->counters, 0, kStaticMaxWorkers * sizeof(int), stream));
     using S = GemmSmem<1, 128, 4, false, 64>;
-    gemm_nvfp4_kernel<1, 128, 4, false, 64><<<grid, kGemmThreads, S::kDynamicBytes, stream>>>(g);
+    gemm_nvfp4_kernel<1, 128, 4, false, 64><<<grid, S::kThreads, S::kDynamicBytes, stream>>>(g);
     CUDA_TRY(cudaGetLastError());
     g_launches.fetch_add(1);
     t_last_kernel = "gemm_1cta_n128_s4_direct(static scratch)";
