@@ -58,30 +58,6 @@ struct DecodeSmem {
     static_assert(kDynamicBytes <= 232448, "exceeds the 227 KB of shared memory one CTA may use");
 };
 
-// bias and activation on 16 columns from output column gcol on, as in gemm_sm100.cuh
-__device__ __forceinline__ void bias_act16(const GemmParams& p, int gcol, float* s) {
-    if (p.bias != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const uint4 b8 = *reinterpret_cast<const uint4*>(p.bias + gcol + 8 * j);
-            const uint32_t w[4] = {b8.x, b8.y, b8.z, b8.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-                s[8 * j + 2 * e] = __fadd_rn(s[8 * j + 2 * e], f.x);
-                s[8 * j + 2 * e + 1] = __fadd_rn(s[8 * j + 2 * e + 1], f.y);
-            }
-        }
-    }
-    if (p.activation == kActRelu) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) s[i] = fmaxf(s[i], 0.f);
-    } else if (p.activation == kActSilu) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) s[i] = __fdividef(s[i], 1.f + __expf(-s[i]));
-    }
-}
-
 // Scale buffers behind the accumulator's BT columns; the double buffers of the two operands.
 constexpr int kDecodeSfwCol = 128, kDecodeSfxCol = 160, kDecodeTmemCols = 256;
 
@@ -271,34 +247,33 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
                 }
                 const int token = ks_rank * S::kPieceTokens + c * S::kChunkTokens + t_in_chunk;
                 if (t_in_chunk < S::kChunkTokens && token < p.M) {
-                    float s[kCols];
+                    // (the extended epilogue's code exists once, for 16 columns a turn: it is fetched cold)
+                    constexpr int kUnroll = EPI_EX ? 1 : kCols / 16;
+#pragma unroll kUnroll
+                    for (int h = 0; h < kCols; h += 16) {
+                        float s[16];
 #pragma unroll
-                    for (int i = 0; i < kCols; ++i) s[i] = 0.f;
+                        for (int i = 0; i < 16; ++i) s[i] = 0.f;
 #pragma unroll
-                    for (int r = 0; r < KS; ++r) {   // ascending rank: the same sum whoever finalises
-                        const float* src = (r == ks_rank) ? stage_gen + token * kBM
-                                                          : land_gen + (r - (r > ks_rank ? 1 : 0)) * (S::kPieceBytes / 4) + (c * S::kChunkTokens + t_in_chunk) * kBM;
+                        for (int r = 0; r < KS; ++r) {   // ascending rank: the same sum whoever finalises
+                            const float* src = (r == ks_rank) ? stage_gen + token * kBM
+                                                              : land_gen + (r - (r > ks_rank ? 1 : 0)) * (S::kPieceBytes / 4) + (c * S::kChunkTokens + t_in_chunk) * kBM;
 #pragma unroll
-                        for (int j = 0; j < kCols / 4; ++j) {
-                            const float4 t = *reinterpret_cast<const float4*>(src + unit_at(token, c0 / 4 + j) * 4);
-                            s[4 * j] += t.x; s[4 * j + 1] += t.y; s[4 * j + 2] += t.z; s[4 * j + 3] += t.w;
+                            for (int j = 0; j < 4; ++j) {
+                                const float4 t = *reinterpret_cast<const float4*>(src + unit_at(token, (c0 + h) / 4 + j) * 4);
+                                s[4 * j] += t.x; s[4 * j + 1] += t.y; s[4 * j + 2] += t.z; s[4 * j + 3] += t.w;
+                            }
                         }
-                    }
-                    if constexpr (EPI_EX) {
-#pragma unroll
-                        for (int h = 0; h < kCols; h += 16) bias_act16(p, gcol + h, &s[h]);
-                    }
-                    if (!EPI_EX || !p.out_nvfp4) {
-                        __half* dst = p.c + l * p.c_batch_stride + static_cast<long long>(token) * p.c_row_stride + gcol;
-#pragma unroll
-                        for (int j = 0; j < kCols / 8; ++j) *reinterpret_cast<uint4*>(dst + 8 * j) = pack8_fp16(&s[8 * j]);
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < kCols; h += 16) {
+                        if constexpr (EPI_EX) bias_act16(p, gcol + h, s);
+                        if (!EPI_EX || !p.out_nvfp4) {
+                            __half* dst = p.c + l * p.c_batch_stride + static_cast<long long>(token) * p.c_row_stride + gcol + h;
+                            *reinterpret_cast<uint4*>(dst) = pack8_fp16(&s[0]);
+                            *reinterpret_cast<uint4*>(dst + 8) = pack8_fp16(&s[8]);
+                        } else {
                             float v[16];
 #pragma unroll
                             for (int i = 0; i < 8; ++i) {   // the fp16-rounded values are quantised, as in gemm_sm100.cuh
-                                const float2 f = __half22float2(__floats2half2_rn(s[h + 2 * i], s[h + 2 * i + 1]));
+                                const float2 f = __half22float2(__floats2half2_rn(s[2 * i], s[2 * i + 1]));
                                 v[2 * i] = f.x;
                                 v[2 * i + 1] = f.y;
                             }

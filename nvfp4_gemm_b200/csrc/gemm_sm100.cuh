@@ -249,6 +249,30 @@ __device__ __forceinline__ uint4 pack8_fp16(const uint32_t* v) {
     return pack8_fp16(f);
 }
 
+// bias and activation on 16 columns from output column gcol on (extended epilogue)
+__device__ __forceinline__ void bias_act16(const GemmParams& p, int gcol, float* s) {
+    if (p.bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint4 b8 = *reinterpret_cast<const uint4*>(p.bias + gcol + 8 * j);
+            const uint32_t w[4] = {b8.x, b8.y, b8.z, b8.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                s[8 * j + 2 * e] = __fadd_rn(s[8 * j + 2 * e], f.x);
+                s[8 * j + 2 * e + 1] = __fadd_rn(s[8 * j + 2 * e + 1], f.y);
+            }
+        }
+    }
+    if (p.activation == kActRelu) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s[i] = fmaxf(s[i], 0.f);
+    } else if (p.activation == kActSilu) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s[i] = __fdividef(s[i], 1.f + __expf(-s[i]));
+    }
+}
+
 template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1, bool EPI_EX = false>
 __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS>::kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ GemmParams p) {
     static_assert(!(EPI_EX && TMA_STORE), "the extended epilogue writes with plain stores");
@@ -573,114 +597,78 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                 *reinterpret_cast<uint4*>(p.c + c_off + col) = q;
                 for (int r = 0; r < p.n_peer; ++r) *reinterpret_cast<uint4*>(p.c_peer[r] + c_off + col) = q;
             };
-            // 32 finished columns [c0, c0 + 32) of this thread's row, fp32: the plain kernels round to
-            // fp16 and store; the extended epilogue adds the bias, applies the activation and writes
-            // fp16 or NVFP4.  The NVFP4 form quantises the fp16-ROUNDED values, so the result equals
-            // the stand-alone quantiser run on the fp16 output.
-            // (extended epilogue) bias and activation on 32 columns starting at global column gcol
-            auto bias_act32 = [&](int gcol, float (&s)[32]) {
-                if (p.bias != nullptr) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint4 b8 = *reinterpret_cast<const uint4*>(p.bias + gcol + 8 * j);
-                        const uint32_t w[4] = {b8.x, b8.y, b8.z, b8.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-                            s[8 * j + 2 * e] = __fadd_rn(s[8 * j + 2 * e], f.x);
-                            s[8 * j + 2 * e + 1] = __fadd_rn(s[8 * j + 2 * e + 1], f.y);
-                        }
-                    }
-                }
-                if (p.activation == kActRelu) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) s[i] = fmaxf(s[i], 0.f);
-                } else if (p.activation == kActSilu) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) s[i] = __fdividef(s[i], 1.f + __expf(-s[i]));
-                }
-            };
-            // 32 values -> 16 bytes of e2m1 codes and the two e4m3 scale bytes (low byte = lower columns)
-            auto quantize32 = [&](const float (&s)[32], uint32_t (&q)[4]) {
-                uint32_t sf2 = 0u;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float v[16];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {   // round to fp16 and back, two at a time
-                        const float2 f = __half22float2(__floats2half2_rn(s[16 * h + 2 * i], s[16 * h + 2 * i + 1]));
-                        v[2 * i] = f.x;
-                        v[2 * i + 1] = f.y;
-                    }
-                    uint32_t o[2];
-                    sf2 |= static_cast<uint32_t>(quantize_block16(v, o)) << (8 * h);
-                    q[2 * h] = o[0];
-                    q[2 * h + 1] = o[1];
-                }
-                return sf2;
-            };
-            auto packed_at = [&](int gcol) {
-                return p.out_packed + l * p.out_packed_batch_stride + static_cast<long long>(row) * p.out_packed_row_stride + gcol / 2;
-            };
-            auto sf_plain_at = [&](int gcol) { return p.out_sf + l * p.out_sf_batch_stride + static_cast<long long>(row) * p.out_sf_row_stride + gcol / 16; };
-            auto sf_perm_at = [&](int gcol) {   // scale of (row, 16-column block gcol / 16) in the 128 x 4 atom layout
-                const int blk = gcol / 16;
-                return p.out_sf_perm + l * p.out_sf_perm_batch_stride + (row / 128) * p.out_sf_perm_block_stride + (blk / 4) * 512 + (row % 32) * 16 +
-                       ((row / 32) % 4) * 4 + (blk % 4);
-            };
-            auto emit32 = [&](int c0, float (&s)[32]) {
+            // Finished columns of this thread's row, fp32: the plain kernels round to fp16 and store; the
+            // extended epilogue adds the bias, applies the activation and writes fp16 or NVFP4.  The
+            // NVFP4 form quantises the fp16-ROUNDED values, so the result equals the stand-alone
+            // quantiser run on the fp16 output.
+            // COLS columns [c0, c0 + COLS), c0 a multiple of COLS = 32 or 64.
+            auto emit = [&](int c0, auto& s) {
+                constexpr int kCols = sizeof(s) / sizeof(float);
                 if constexpr (!EPI_EX) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) store8(c0 + 8 * j, pack8_fp16(&s[8 * j]));
+                    for (int j = 0; j < kCols / 8; ++j) store8(c0 + 8 * j, pack8_fp16(&s[8 * j]));
                 } else {
+                    // Sixteen columns (a scale block) a turn, the rest moved up: the code of a block exists
+                    // once.  Codes and scales of the NVFP4 form are collected and stored together: 64
+                    // columns are 32 bytes of codes (one full sector) and the four scales of one unit of either layout.
                     const int gcol = nb * BN + c0;
-                    bias_act32(gcol, s);
-                    if (!p.out_nvfp4) {
+                    uint32_t q[kCols / 8];
+                    uint32_t sf = 0u;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) store8(c0 + 8 * j, pack8_fp16(&s[8 * j]));
-                    } else {
-                        uint32_t q[4];
-                        const uint16_t sf2 = static_cast<uint16_t>(quantize32(s, q));   // two scales: neighbours in both layouts
-                        *reinterpret_cast<uint4*>(packed_at(gcol)) = make_uint4(q[0], q[1], q[2], q[3]);
-                        if (p.out_sf != nullptr) *reinterpret_cast<uint16_t*>(sf_plain_at(gcol)) = sf2;
-                        if (p.out_sf_perm != nullptr) *reinterpret_cast<uint16_t*>(sf_perm_at(gcol)) = sf2;
-                    }
-                }
-            };
-            // 64 columns [c0, c0 + 64), c0 a multiple of 64.  The NVFP4 form then has 32 bytes of codes
-            // (one full sector) and the four scales of one unit of either scale layout: one store
-            // each where the addresses allow it, instead of twice two partial ones.
-            auto emit64 = [&](int c0, float (&sa)[32], float (&sb)[32]) {
-                if constexpr (!EPI_EX) {
-                    emit32(c0, sa);
-                    emit32(c0 + 32, sb);
-                } else {
-                    if (!p.out_nvfp4) {
-                        emit32(c0, sa);
-                        emit32(c0 + 32, sb);
-                        return;
-                    }
-                    const int gcol = nb * BN + c0;
-                    bias_act32(gcol, sa);
-                    bias_act32(gcol + 32, sb);
-                    uint32_t qa[4], qb[4];
-                    const uint32_t sf4 = quantize32(sa, qa) | (quantize32(sb, qb) << 16);
-                    uint8_t* dst = packed_at(gcol);
-                    if (wide_packed) {
-                        ptx::st_global_32B(dst, qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3]);
-                    } else {
-                        *reinterpret_cast<uint4*>(dst) = make_uint4(qa[0], qa[1], qa[2], qa[3]);
-                        *reinterpret_cast<uint4*>(dst + 16) = make_uint4(qb[0], qb[1], qb[2], qb[3]);
-                    }
-                    if (p.out_sf != nullptr) {
-                        if (wide_sf) {
-                            *reinterpret_cast<uint32_t*>(sf_plain_at(gcol)) = sf4;
+                    for (int i = 0; i < kCols / 8; ++i) q[i] = 0u;
+#pragma unroll 1
+                    for (int h = 0; h < kCols; h += 16) {
+                        bias_act16(p, gcol + h, s);
+                        if (!p.out_nvfp4) {
+                            store8(c0 + h, pack8_fp16(&s[0]));
+                            store8(c0 + h + 8, pack8_fp16(&s[8]));
                         } else {
-                            *reinterpret_cast<uint16_t*>(sf_plain_at(gcol)) = static_cast<uint16_t>(sf4);
-                            *reinterpret_cast<uint16_t*>(sf_plain_at(gcol + 32)) = static_cast<uint16_t>(sf4 >> 16);
+                            float v[16];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {   // round to fp16 and back, two at a time
+                                const float2 f = __half22float2(__floats2half2_rn(s[2 * i], s[2 * i + 1]));
+                                v[2 * i] = f.x;
+                                v[2 * i + 1] = f.y;
+                            }
+                            uint32_t o[2];
+                            sf |= static_cast<uint32_t>(quantize_block16(v, o)) << (h / 2);
+#pragma unroll
+                            for (int i = 0; i + 2 < kCols / 8; ++i) q[i] = q[i + 2];
+                            q[kCols / 8 - 2] = o[0];
+                            q[kCols / 8 - 1] = o[1];
+                        }
+#pragma unroll
+                        for (int i = 0; i + 16 < kCols; ++i) s[i] = s[i + 16];
+                    }
+                    if (p.out_nvfp4) {
+                        const int blk = gcol / 16;
+                        uint8_t* dst = p.out_packed + l * p.out_packed_batch_stride + static_cast<long long>(row) * p.out_packed_row_stride + gcol / 2;
+                        uint8_t* sf_plain = p.out_sf + l * p.out_sf_batch_stride + static_cast<long long>(row) * p.out_sf_row_stride + blk;
+                        // scale of (row, block) in the 128 x 4 atom layout
+                        uint8_t* sf_perm = p.out_sf_perm + l * p.out_sf_perm_batch_stride + (row / 128) * p.out_sf_perm_block_stride + (blk / 4) * 512 +
+                                           (row % 32) * 16 + ((row / 32) % 4) * 4 + (blk % 4);
+                        if constexpr (kCols == 64) {
+                            if (wide_packed) {
+                                ptx::st_global_32B(dst, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
+                            } else {
+                                *reinterpret_cast<uint4*>(dst) = make_uint4(q[0], q[1], q[2], q[3]);
+                                *reinterpret_cast<uint4*>(dst + 16) = make_uint4(q[4], q[5], q[6], q[7]);
+                            }
+                            if (p.out_sf != nullptr) {
+                                if (wide_sf) {
+                                    *reinterpret_cast<uint32_t*>(sf_plain) = sf;
+                                } else {
+                                    *reinterpret_cast<uint16_t*>(sf_plain) = static_cast<uint16_t>(sf);
+                                    *reinterpret_cast<uint16_t*>(sf_plain + 2) = static_cast<uint16_t>(sf >> 16);
+                                }
+                            }
+                            if (p.out_sf_perm != nullptr) *reinterpret_cast<uint32_t*>(sf_perm) = sf;   // (16-byte aligned atoms: always aligned)
+                        } else {
+                            *reinterpret_cast<uint4*>(dst) = make_uint4(q[0], q[1], q[2], q[3]);
+                            if (p.out_sf != nullptr) *reinterpret_cast<uint16_t*>(sf_plain) = static_cast<uint16_t>(sf);
+                            if (p.out_sf_perm != nullptr) *reinterpret_cast<uint16_t*>(sf_perm) = static_cast<uint16_t>(sf);
                         }
                     }
-                    if (p.out_sf_perm != nullptr) *reinterpret_cast<uint32_t*>(sf_perm_at(gcol)) = sf4;   // (16-byte aligned atoms: always aligned)
                 }
             };
             auto release_acc = [&]() {
@@ -823,7 +811,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                             }
                         }
                     }
-                    if (row < p.M) emit32(ks_rank * kMyCols + c0, s);
+                    if (row < p.M) emit(ks_rank * kMyCols + c0, s);
                 }
                 release_acc();
             } else if (TMA_STORE && whole_tile) {
@@ -920,24 +908,16 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                                           make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
                     };
-                    if constexpr (kAccOverlap) {
-                        uint32_t held[kMyRelease][32];
-#pragma unroll
-                        for (int pos = 0; pos < kMyRelease; ++pos) ptx::tc_ld_32cols(t_acc + my_chunk(pos) * 32, held[pos]);
-                        ptx::tc_wait_ld();
-                        release_acc();  // the MMA warp may start the next tile now
-#pragma unroll
-                        for (int pos = 0; pos < kMyRelease; ++pos) publish32(my_chunk(pos) * 32, held[pos]);
-                    }
 #pragma unroll 1
-                    for (int pos = kAccOverlap ? kMyRelease : 0; pos < kMyChunks; ++pos) {
-                        const int c0 = my_chunk(pos) * 32;
-                        uint32_t v[32];
-                        ptx::tc_ld_32cols(t_acc + c0, v);
+                    for (int i = 0; i < kMyChunks; i += 2) {
+                        uint32_t va[32], vb[32];
+                        ptx::tc_ld_32cols(t_acc + my_chunk(i) * 32, va);
+                        ptx::tc_ld_32cols(t_acc + my_chunk(i + 1) * 32, vb);
                         ptx::tc_wait_ld();
-                        publish32(c0, v);
+                        if (i == 0) release_acc();  // the MMA warp may start the next tile now
+                        publish32(my_chunk(i) * 32, va);
+                        publish32(my_chunk(i + 1) * 32, vb);
                     }
-                    if constexpr (!kAccOverlap) release_acc();
                     __threadfence();
                     ptx::named_bar_sync(1, kEpiThreads);
                     if (epi_tid == 0) atomicAdd(counter, k1 - k0);
@@ -949,67 +929,58 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                     // contributor (64 registers) are requested before anything is added.
                     const int w_last = whole_tile ? w_first : unit_owner(tile * KT + KT - 1, n_workers, p.total_units);
                     const int need = KT - (k1 - k0);
-                    // Everything the hand-back waits for goes to registers first (the half an
-                    // overlapped accumulator shares with the other one, else all of it: two
-                    // 32-column pieces per thread), the accumulator is released, and only then anything is
-                    // waited for, converted or stored.
-                    uint32_t held[kMyRelease][32];
+                    // 64 columns at a time, in ONE copy of the code: a launch that follows another kernel
+                    // fetches it cold, line by line through L2.  (Unrolled over the tile and over the scale
+                    // blocks of a step, the re-quantising form with SiLU took 17 us longer after another
+                    // kernel than after itself.)  What the hand-back waits for is the first step's: it goes to
+                    // registers, the accumulator is released, and only then anything is waited for, converted or stored.
+                    static_assert(kMyRelease == 2 && kMyChunks % 2 == 0, "the hand-back follows the first 64 columns");
+                    bool ready = true;
+#pragma unroll 1
+                    for (int i = 0; i < kMyChunks; i += 2) {
+                        const int c0 = my_chunk(i) * 32;             // (my_chunk(i + 1) is the neighbour)
+                        float s[64];
+                        {
+                            uint32_t va[32], vb[32];
+                            ptx::tc_ld_32cols(t_acc + c0, va);
+                            ptx::tc_ld_32cols(t_acc + c0 + 32, vb);
+                            ptx::tc_wait_ld();
 #pragma unroll
-                    for (int pos = 0; pos < kMyRelease; ++pos) ptx::tc_ld_32cols(t_acc + my_chunk(pos) * 32, held[pos]);
-                    ptx::tc_wait_ld();
-                    release_acc();
-                    if (!whole_tile) {
-                        bool ready = true;
-                        if (epi_tid == 0) {
-                            const long long t_spin = clock64();
-                            while (ptx::ld_acquire_gpu(counter) < need) {
-                                if (*abort_flag || static_cast<uint64_t>(clock64() - t_spin) > timeout) {
-                                    *abort_flag = 1u;
-                                    ready = false;
-                                    break;
+                            for (int e = 0; e < 32; ++e) { s[e] = __uint_as_float(va[e]); s[32 + e] = __uint_as_float(vb[e]); }
+                        }
+                        if (i == 0) {
+                            release_acc();
+                            if (!whole_tile) {
+                                if (epi_tid == 0) {
+                                    const long long t_spin = clock64();
+                                    while (ptx::ld_acquire_gpu(counter) < need) {
+                                        if (*abort_flag || static_cast<uint64_t>(clock64() - t_spin) > timeout) {
+                                            *abort_flag = 1u;
+                                            ready = false;
+                                            break;
+                                        }
+                                        __nanosleep(64);
+                                    }
                                 }
-                                __nanosleep(64);
+                                ready = ptx::named_bar_and(1, kEpiThreads, ready);
+                                if (!ready) break;
                             }
                         }
-                        if (!ptx::named_bar_and(1, kEpiThreads, ready)) break;
-                    }
-                    static_assert(kMyChunks % 2 == 0 && kMyRelease % 2 == 0, "the partial sums are added 64 columns at a time");
-                    // the columns [c0a, c0a + 32) and [c0b, c0b + 32) of this thread's row: own sums in, total out
-                    auto add_others_and_emit = [&](int c0a, int c0b, float (&sa)[32], float (&sb)[32]) {
 #pragma unroll 1
                         for (int w = w_first + 1; w <= w_last; ++w) {   // later contributors use their "head" slot
                             const float* src = p.scratch + static_cast<long long>(partial_slot(w, 1, CG, cta_rank)) * (kBM * BN) + row_in_tile * 4;
-                            float4 ta[8], tb[8];
+                            float4 t[16];
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) ta[j] = ptx::ld_cg_v4(src + (c0a / 4 + j) * (kBM * 4));
+                            for (int j = 0; j < 16; ++j) t[j] = ptx::ld_cg_v4(src + (c0 / 4 + j) * (kBM * 4));
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) tb[j] = ptx::ld_cg_v4(src + (c0b / 4 + j) * (kBM * 4));
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                sa[4 * j] += ta[j].x; sa[4 * j + 1] += ta[j].y; sa[4 * j + 2] += ta[j].z; sa[4 * j + 3] += ta[j].w;
-                                sb[4 * j] += tb[j].x; sb[4 * j + 1] += tb[j].y; sb[4 * j + 2] += tb[j].z; sb[4 * j + 3] += tb[j].w;
+                            for (int j = 0; j < 16; ++j) {
+                                s[4 * j] += t[j].x; s[4 * j + 1] += t[j].y; s[4 * j + 2] += t[j].z; s[4 * j + 3] += t[j].w;
                             }
                         }
-                        if (row < p.M) emit64(c0a, sa, sb);   // (c0b == c0a + 32: drain positions pair up neighbouring chunks)
-                    };
-#pragma unroll
-                    for (int pos = 0; pos < kMyRelease; pos += 2) {
-                        float sa[32], sb[32];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) { sa[i] = __uint_as_float(held[pos][i]); sb[i] = __uint_as_float(held[pos + 1][i]); }
-                        add_others_and_emit(my_chunk(pos) * 32, my_chunk(pos + 1) * 32, sa, sb);
+                        if (row < p.M) emit(c0, s);
+                        __syncwarp();
                     }
-#pragma unroll 1
-                    for (int pos = kMyRelease; pos < kMyChunks; pos += 2) {
-                        uint32_t va[32], vb[32];
-                        ptx::tc_ld_32cols(t_acc + my_chunk(pos) * 32, va);
-                        ptx::tc_ld_32cols(t_acc + my_chunk(pos + 1) * 32, vb);
-                        ptx::tc_wait_ld();
-                        float sa[32], sb[32];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) { sa[i] = __uint_as_float(va[i]); sb[i] = __uint_as_float(vb[i]); }
-                        add_others_and_emit(my_chunk(pos) * 32, my_chunk(pos + 1) * 32, sa, sb);
-                    }
+                    if (!ready) break;
                     if (!whole_tile && epi_tid == 0) *counter = 0;
                 }
             }
