@@ -1,4 +1,4 @@
-// NVFP4 GEMM for at most 128 rows of activations (decode):  C[M,N] (fp16) = (A x SFA) . (B x SFB)^T.
+// NVFP4 GEMM for few rows of activations (decode; up to 128, a few times 128 with K split):  C[M,N] (fp16) = (A x SFA) . (B x SFB)^T.
 //
 // Operands are swapped on the tensor core: the weights B are the M operand (128 of their rows = output
 // columns per CTA), the activations A the N operand, BT = 32, 64 or 128 of them.  D[column, token]
@@ -107,8 +107,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
     }
     const int KT = p.k_tiles;
     const int tile = static_cast<int>(blockIdx.x) / KS;
-    const int l = tile / p.tiles_n;
-    const int nb = tile - l * p.tiles_n;   // 128-row block of the weights
+    // (the token tiles that share a block of weights are neighbours, so that it comes from HBM once)
+    const int mt = tile % p.tiles_m;                 // token tile
+    const int l = tile / p.tiles_m / p.tiles_n;
+    const int nb = tile / p.tiles_m - l * p.tiles_n; // 128-row block of the weights
     const int k0 = (ks_rank * KT) / KS, k1 = ((ks_rank + 1) * KT) / KS;
     const uint64_t timeout = p.timeout_cycles;
     // the first operands are asked into L2 ahead of the dependency wait (see gemm_sm100.cuh)
@@ -117,8 +119,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
             for (int kt = k0; kt < min(k1, k0 + kPrefetchStages); ++kt) {
                 ptx::tma_prefetch_3d(&p.tma_b, kt * kBKBytes, nb * kBM, l);
                 ptx::tma_prefetch_4d(&p.tma_sfb, 0, kt * kMmaPerStage, nb, l);
-                ptx::tma_prefetch_3d(&p.tma_a, kt * kBKBytes, 0, l);
-                ptx::tma_prefetch_4d(&p.tma_sfa, 0, kt * kMmaPerStage, 0, l);
+                ptx::tma_prefetch_3d(&p.tma_a, kt * kBKBytes, mt * BT, l);
+                ptx::tma_prefetch_4d(&p.tma_sfa, 0, kt * kMmaPerStage, mt, l);
             }
         }
         __syncwarp();
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         const uint64_t pol_x = ptx::policy_evict_last();     // re-read by every weight block
-        const uint64_t pol_w = ptx::policy_evict_first();    // streams through once
+        const uint64_t pol_w = p.tiles_m > 1 ? ptx::policy_evict_last() : ptx::policy_evict_first();   // read once per token tile
         if (ptx::elect_one()) {
             uint32_t stage = 0, phase = 0;
             for (int kt = k0; kt < k1; ++kt) {
@@ -146,8 +148,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
                 ptx::mbar_expect_tx(full, S::kStageBytes);
                 ptx::tma_load_3d(sw, &p.tma_b, kt * kBKBytes, nb * kBM, l, full, pol_w);
                 ptx::tma_load_4d(ssfw, &p.tma_sfb, 0, kt * kMmaPerStage, nb, l, full);
-                ptx::tma_load_3d(sx, &p.tma_a, kt * kBKBytes, 0, l, full, pol_x);
-                ptx::tma_load_4d(ssfx, &p.tma_sfa, 0, kt * kMmaPerStage, 0, l, full);
+                ptx::tma_load_3d(sx, &p.tma_a, kt * kBKBytes, mt * BT, l, full, pol_x);
+                ptx::tma_load_4d(ssfx, &p.tma_sfa, 0, kt * kMmaPerStage, mt, l, full);
                 if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             }
         }
@@ -245,8 +247,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
                     ok = ptx::mbar_wait_bounded<true>(bar_land + c * 8, 0u, abort_flag, timeout);
                     if (!ptx::named_bar_and(2, 128, ok)) break;
                 }
-                const int token = ks_rank * S::kPieceTokens + c * S::kChunkTokens + t_in_chunk;
-                if (t_in_chunk < S::kChunkTokens && token < p.M) {
+                const int token = ks_rank * S::kPieceTokens + c * S::kChunkTokens + t_in_chunk;   // in the tile
+                const int row = mt * BT + token;
+                if (t_in_chunk < S::kChunkTokens && row < p.M) {
                     // (the extended epilogue's code exists once, for 16 columns a turn: it is fetched cold)
                     constexpr int kUnroll = EPI_EX ? 1 : kCols / 16;
 #pragma unroll kUnroll
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
                         }
                         if constexpr (EPI_EX) bias_act16(p, gcol + h, s);
                         if (!EPI_EX || !p.out_nvfp4) {
-                            __half* dst = p.c + l * p.c_batch_stride + static_cast<long long>(token) * p.c_row_stride + gcol + h;
+                            __half* dst = p.c + l * p.c_batch_stride + static_cast<long long>(row) * p.c_row_stride + gcol + h;
                             *reinterpret_cast<uint4*>(dst) = pack8_fp16(&s[0]);
                             *reinterpret_cast<uint4*>(dst + 8) = pack8_fp16(&s[8]);
                         } else {
@@ -280,11 +283,11 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
                             uint32_t o[2];
                             const uint8_t sf = quantize_block16(v, o);
                             const int blk = (gcol + h) / 16;
-                            *reinterpret_cast<uint2*>(p.out_packed + l * p.out_packed_batch_stride + static_cast<long long>(token) * p.out_packed_row_stride +
+                            *reinterpret_cast<uint2*>(p.out_packed + l * p.out_packed_batch_stride + static_cast<long long>(row) * p.out_packed_row_stride +
                                                       blk * 8) = make_uint2(o[0], o[1]);
-                            if (p.out_sf != nullptr) p.out_sf[l * p.out_sf_batch_stride + static_cast<long long>(token) * p.out_sf_row_stride + blk] = sf;
-                            if (p.out_sf_perm != nullptr)   // (tokens < 128: one row block)
-                                p.out_sf_perm[l * p.out_sf_perm_batch_stride + (blk / 4) * 512 + (token % 32) * 16 + (token / 32) * 4 + blk % 4] = sf;
+                            if (p.out_sf != nullptr) p.out_sf[l * p.out_sf_batch_stride + static_cast<long long>(row) * p.out_sf_row_stride + blk] = sf;
+                            if (p.out_sf_perm != nullptr)   // (more than one token tile: of 128, a row block each)
+                                p.out_sf_perm[l * p.out_sf_perm_batch_stride + mt * p.out_sf_perm_block_stride + (blk / 4) * 512 + (token % 32) * 16 + (token / 32) * 4 + blk % 4] = sf;
                         }
                     }
                 }
@@ -292,8 +295,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
             }
             if constexpr (EPI_EX) {
                 // rows of the 128-row scale block that do not exist read as zero scales: eight blocks = two words per row
-                if (p.out_nvfp4 && p.out_sf_perm != nullptr && ks_rank == 0 && tid >= p.M) {
-                    uint8_t* dst = p.out_sf_perm + l * p.out_sf_perm_batch_stride + nb * 2 * 512 + (tid % 32) * 16 + (tid / 32) * 4;
+                if (p.out_nvfp4 && p.out_sf_perm != nullptr && ks_rank == 0 && mt * BT + tid >= p.M) {
+                    uint8_t* dst = p.out_sf_perm + l * p.out_sf_perm_batch_stride + mt * p.out_sf_perm_block_stride + nb * 2 * 512 + (tid % 32) * 16 + (tid / 32) * 4;
                     *reinterpret_cast<uint32_t*>(dst) = 0u;
                     *reinterpret_cast<uint32_t*>(dst + 512) = 0u;
                 }

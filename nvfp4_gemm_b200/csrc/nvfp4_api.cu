@@ -363,7 +363,7 @@ int launch_gemm_decode(const DeviceCtx* c, const GemmParams& params, bool epi, c
     }
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(params.tiles_n * params.L * KS, 1, 1);
+    cfg.gridDim = dim3(params.tiles_m * params.tiles_n * params.L * KS, 1, 1);
     cfg.blockDim = dim3(kDecodeThreads, 1, 1);
     cfg.dynamicSmemBytes = S::kDynamicBytes;
     cfg.stream = stream;
@@ -477,23 +477,26 @@ struct DecodeChoice {
 // exchange (0.3-1 us) and pays when the k-tiles it takes off each CTA cost more:
 //   * 8 CTAs per tile only for up to eight tiles (clusters of eight do not fit side by side: 16 tiles run in
 //     two waves, 11.4 against 6.9 us) and K >= 12288 (17 x 512 x 16384: 5.05 us, four 5.94; x 7168: 4.03, 4.09);
-//   * 4 when they fit one wave: up to half a wave from K = 2048 (17 x 2048 x 2048: 3.31 us, unsplit 3.50),
+//   * 4 when they fit one wave (clusters of four leave SMs of a GPC over: 32 fit 148 SMs, 36 tiles ran in two
+//     waves, 15.2 against 8.2 us): up to half a wave from K = 2048 (17 x 2048 x 2048: 3.31 us, unsplit 3.50),
 //     else from K = 6144 (17 x 4096 x 7168: 5.91, two 6.20; x 4096: 4.90, 4.92; 128 rows 6.77, 6.52);
 //   * 2 when they fit one wave: up to half a wave from K = 3072 (17 x 4096 x 4096: 4.92, unsplit
 //     5.33; x 2048: 3.89, 3.85), else from K = 6144 (17 x 7168 x 7168: 7.48, unsplit 7.87; x 4096: 5.79, 5.72).
 // More than 64 rows run here only when K is split (unsplit the 128-row-tile kernel is as fast or faster), so
 // two pays earlier: from K = 4096 on a whole wave (128 x 7168 x 4096: 7.38, 7.73 unsplit), and four from 3072.
+// More than 128 rows are several token tiles of 128, under the same rules: 256 x 1536 x 16384 takes 8.9 us (unsplit
+// 128 x 128 tiles 16.2, shared tiles 22.7), 256 x 4096 x 7168 8.2 (9.6), 384 x 1536 x 7168 6.8 (8.2).
 // More tiles than SMs: two CTAs per SM, so that one's start and end hide behind the other
 // (17 x 28672 x 2048: 7.07 against 9.29 us); up to one wave the deep ring is ahead (12288 columns: 4.55, 5.07).
 DecodeChoice choose_decode(int m, int n, int k, int l, int num_sms, const nvfp4_gemm_config& cf) {
-    if (m > kBM || cf.cta_group == 2 || cf.tile_n != 0 || cf.grid != 0 || cf.split_k != 0 || cf.epilogue != 0) return DecodeChoice{0, 0, false};
+    if (cf.cta_group == 2 || cf.tile_n != 0 || cf.grid != 0 || cf.split_k != 0 || cf.epilogue != 0) return DecodeChoice{0, 0, false};
     const int tokens = m <= 32 ? 32 : m <= 64 ? 64 : 128;
-    const long long tiles = static_cast<long long>(n / kBM) * l;
+    const long long tiles = static_cast<long long>((m + kBM - 1) / kBM) * (n / kBM) * l;
     const int k_tiles = k / kKPerStage;
     const bool wide = tokens == 128;
     int split = 1;
     if (tiles <= 8 && k_tiles >= 48) split = 8;
-    else if (tiles * 4 <= num_sms && k_tiles >= (tiles * 8 <= num_sms ? (wide ? 12 : 8) : 24)) split = 4;
+    else if (tiles * 32 <= num_sms * 7LL && k_tiles >= (tiles * 8 <= num_sms ? (wide ? 12 : 8) : 24)) split = 4;
     else if (tiles * 2 <= num_sms && k_tiles >= (tiles * 4 <= num_sms ? 12 : wide ? 16 : 24)) split = 2;
     if (wide && split == 1) split = 0;
     return DecodeChoice{tokens, split, split == 1 && tiles > num_sms};
@@ -644,7 +647,7 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
 
     const DecodeChoice decode = choose_decode(p->m, p->n, p->k, p->l, c->num_sms, cf);
     if (decode.split > 0 && n_peers == 0) {
-        g.tiles_m = 1;
+        g.tiles_m = (p->m + decode.tokens - 1) / decode.tokens;
         g.tiles_n = p->n / kBM;
         if (int rc = encode_map(make_key(p->a, kbytes, p->m, p->l, p->a_row_stride, a_bs, kBKBytes, decode.tokens, CU_TENSOR_MAP_DATA_TYPE_UINT8),
                              &g.tma_a)) return rc;

@@ -1,4 +1,4 @@
-"""The decode kernel (at most 128 rows): every tile width, split of K and ring depth, at the edges of its tiles."""
+"""The decode kernel (few rows): every tile width, split of K and ring depth, at the edges of its tiles."""
 import pytest
 import torch
 
@@ -16,6 +16,7 @@ CASES = [
     ((40, 6400, 512, 3), "gemm_decode_t64_s3"), ((64, 19072, 1280, 1), "gemm_decode_t64_s3"),
     ((65, 2560, 3072, 1), "gemm_splitk2_decode_t128"), ((128, 2432, 4352, 2), "gemm_splitk2_decode_t128"),
     ((97, 256, 3328, 2), "gemm_splitk4_decode_t128"), ((127, 128, 12288, 1), "gemm_splitk8_decode_t128"), ((128, 256, 12544, 1), "gemm_splitk8_decode_t128"),
+    ((129, 1280, 4096, 1), "gemm_splitk2_decode_t128"), ((300, 384, 3072, 2), "gemm_splitk4_decode_t128"), ((256, 128, 12288, 4), "gemm_splitk8_decode_t128"),
 ]
 
 
@@ -61,8 +62,10 @@ def test_decode_epilogue_equals_the_persistent_kernels(sub, shape, kernel):
     assert "decode" not in sub.last_kernel()
     for g, e in zip(got, exp):
         assert torch.equal(g.view(torch.uint8), e.view(torch.uint8)), f"{shape} {kernel}"
-    flat = torch.as_strided(got[2].view(torch.uint8), (l, n // 64, 32, 4, 4), (n // 64 * 512, 512, 16, 4, 1))   # [l][atom][row % 32][row / 32][scale]
-    rows = flat.permute(0, 3, 2, 1, 4).reshape(l, 128, n // 16)
+    blocks = (m + 127) // 128
+    flat = torch.as_strided(got[2].view(torch.uint8), (l, blocks, n // 64, 32, 4, 4),       # [l][row block][atom][row % 32][row / 32][scale]
+                            (blocks * n // 64 * 512, n // 64 * 512, 512, 16, 4, 1))
+    rows = flat.permute(0, 1, 4, 3, 2, 5).reshape(l, blocks * 128, n // 16)
     assert int(rows[:, m:].sum()) == 0
 
 
