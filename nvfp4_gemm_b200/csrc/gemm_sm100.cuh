@@ -575,10 +575,9 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
             const uint32_t acc_phase = (acc_it / kNumAcc) & 1u;
             // All epilogue threads take the same branch: the outcome of the wait is agreed on
             // through a barrier, so a thread that gave up cannot strand the others at a later one.
-            bool got_acc;
-            {
-                got_acc = ptx::mbar_wait_bounded(bar_acc_full + acc * 8, acc_phase, abort_flag, timeout);
-            }
+            // One warp polls; the others sleep in the barrier below (a polling warp costs power, and with it clock).
+            bool got_acc = true;
+            if (warp == 2) got_acc = ptx::mbar_wait_bounded(bar_acc_full + acc * 8, acc_phase, abort_flag, timeout);
             if (!ptx::named_bar_and(2, kEpiThreads, got_acc)) break;
             ptx::tc_fence_after();
             const uint32_t t_acc = tmem_base + acc * S::kAccStride + (static_cast<uint32_t>(quad * 32) << 16);

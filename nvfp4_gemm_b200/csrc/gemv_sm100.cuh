@@ -1,7 +1,7 @@
 // NVFP4 block-scaled GEMV for sm_100a (CUDA cores; the op is HBM-bound, not a dense contraction):
 //   c[m, l] = sum_k  e2m1(a[m,k,l]) * sfa[m,k/16,l] * e2m1(b[k,l]) * sfb[k/16,l]
 //
-// gemv_nvfp4_kernel (K beyond 16384, or a launch shape the caller asks for): one warp streams R rows; a lane owns 32-byte chunks (64 elements = 4 scale blocks) at a
+// gemv_nvfp4_kernel (the other K, or a launch shape the caller asks for): one warp streams R rows; a lane owns 32-byte chunks (64 elements = 4 scale blocks) at a
 // stride of 1024 bytes, so every warp-wide 256-bit load covers 1 KiB of contiguous row.  Per
 // 16-element block the products are summed in f16x2 (8 terms per half: exact), widened to fp32,
 // scaled by sfa*sfb and accumulated in fp32.  The vector and its scales are re-read through L1
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_nvfp4_kernel(const GemvPara
     }
 }
 
-// The form for K up to 16384: the vector stays in registers.  A row worker is LANES lanes (or, for K
+// The form for K up to 8192, and 14400 to 16384: the vector stays in registers.  A row worker is LANES lanes (or, for K
 // beyond 2048, k_warps whole warps side by side), a 64-element chunk of K per lane: it converts its
 // chunks of the vector once and walks rows of the matrix, four at a time with the next four in flight.
 // The matrix is then all that is loaded and converted, where the form above converts the vector again for

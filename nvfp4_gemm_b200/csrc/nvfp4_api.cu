@@ -782,21 +782,26 @@ int nvfp4_gemv_config(const nvfp4_problem* p, int rows_per_warp, int warps_per_c
     if (int rc = gemv_prepare(p, &g)) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 
-    // Up to K = 16384 the vector fits the registers of the warps that share a row.  Lanes per row: as many
+    // The vector fits the registers of the warps that share a row.  Lanes per row: as many
     // as it has 64-element chunks, rounded up to 8, 16 or 32 (more lanes would idle: 28672 x 512 x 8 took 48.4 us
     // with a warp per row and 15.3 with 8 lanes), and no more CTAs than have a whole step of rows to do
     // (2000 x 1024 x 8: 4.8 -> 3.7 us).
     const long long rows_total = static_cast<long long>(p->m) * p->l;
     const int chunks = p->k / 64;
-    if (rows_per_warp == 0 && warps_per_cta == 0 && chunks <= kGemvMaxKWarps * kGemvSliceChunks && rows_total < (1 << 30)) {
+    // Between 8192 and 14336 five to seven warps share a row, which leaves lanes or warps of the SM idle: the other
+    // kernel is as fast or faster there (9000 x 12288 x 3: 32.3 us against 35.3; x 10240: 28.3, 28.3; x 14400: 41.2, 40.3).
+    const int k_warps = (chunks + kGemvSliceChunks - 1) / kGemvSliceChunks;
+    if (rows_per_warp == 0 && warps_per_cta == 0 && (k_warps <= 4 || k_warps == kGemvMaxKWarps) && rows_total < (1 << 30)) {
         DeviceCtx* c = nullptr;
         if (int rc = get_ctx(&c)) return rc;
-        const int k_warps = (chunks + kGemvSliceChunks - 1) / kGemvSliceChunks;
-        const int row_workers = kGemvMaxKWarps / k_warps;
+        // 128 registers a thread let 16 warps share an SM.  Three warps or more per row make a CTA of their own, so that
+        // as many of the 16 as possible are used (28672 x 4992: 19.9 us on 12 warps, 18.2 on 15).
+        const int row_workers = k_warps <= 2 ? kGemvMaxKWarps / k_warps : 1;
+        const int ctas_per_sm = 16 / (k_warps * row_workers);
         const int lanes = chunks <= 8 ? 8 : chunks <= 16 ? 16 : 32;
         const long long step_rows = static_cast<long long>(row_workers) * kGemvRowsPerStep * (32 / lanes);   // one step of a CTA
         long long ctas = (rows_total + step_rows - 1) / step_rows;
-        if (ctas > 2LL * c->num_sms) ctas = 2LL * c->num_sms;      // two fit an SM (128 registers x 256 threads)
+        if (ctas > static_cast<long long>(ctas_per_sm) * c->num_sms) ctas = static_cast<long long>(ctas_per_sm) * c->num_sms;
         cudaLaunchConfig_t cfg;
         std::memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
