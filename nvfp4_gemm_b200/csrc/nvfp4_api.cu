@@ -235,8 +235,11 @@ bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) %
 
 // Whole tiles per worker, or an even split of all (tile, k-tile) units with shared tiles summed
 // through scratch?  In k-tiles of run time: whole tiles cost waves x k_tiles; the even split costs
-// units / workers plus the summing, which hides behind later whole tiles when a worker has at
-// least two tiles' worth of units and otherwise ends the launch (publish, wait, read back:
+// units / workers plus the summing, which hides in part behind later whole tiles when a worker has at
+// least two tiles' worth of units (measured as 13 to 18 k-tiles on ten shapes with 192 to 320 tiles of 256 x 256 and
+// K 2048 to 8192, whole tiles against the split: 4096 x 4096 x 2048 20.8 us against 26.9, 3072 x 4096 x 4096
+// 24.1 against 27.2, 2048 x 7168 x 7168 49.8 against 44.9; counted as 16) and otherwise ends the launch
+// (publish, wait, read back:
 // measured about as long as 24 k-tiles of the 256-wide pair kernel with two workers per tile --
 // 768 x 4096 x 4096 took 19.5 us split 74 ways and 10.6 us as 48 whole tiles -- and counted as 12
 // k-tiles per worker that shares a tile).
@@ -251,7 +254,7 @@ WorkSplit plan_work_split(long long tiles, int k_tiles, int max_workers) {
     const double cost_whole = static_cast<double>(waves) * k_tiles;
     const double share = static_cast<double>(tiles) * k_tiles / max_workers;
     const double per_tile = static_cast<double>(k_tiles) / (share < 1.0 ? 1.0 : share);   // workers that share a tile, about
-    const double cost_split = share + (share >= 2.0 * k_tiles ? 3.0 : 12.0 * (per_tile < 2.0 ? 2.0 : per_tile));
+    const double cost_split = share + (share >= 2.0 * k_tiles ? 16.0 : 12.0 * (per_tile < 2.0 ? 2.0 : per_tile));
     if (cost_whole <= cost_split) return WorkSplit{cost_whole, static_cast<int>((tiles + waves - 1) / waves), true};   // the fewest workers that need no more waves
     return WorkSplit{cost_split, max_workers, false};
 }
@@ -488,6 +491,10 @@ struct DecodeChoice {
 // 128 x 128 tiles 16.2, shared tiles 22.7), 256 x 4096 x 7168 8.2 (9.6), 384 x 1536 x 7168 6.8 (8.2).
 // More tiles than SMs: two CTAs per SM, so that one's start and end hide behind the other
 // (17 x 28672 x 2048: 7.07 against 9.29 us); up to one wave the deep ring is ahead (12288 columns: 4.55, 5.07).
+// With many tiles per SM the persistent kernels, which overlap one tile's stores with the next one's
+// loads, catch up: beyond four waves with K < 1024 (17 x 28672 x 512 x 4: 11.1 us here, 9.4 there; x 1024:
+// 15.0, 17.9) and, as their 256-wide tiles waste less on 64 tokens, beyond two waves with more than 32
+// (50 x 28672 x 1024 x 2: 10.0, 9.2; 50 x 28672 x 512 x 8: 25.2, 15.3; one wave and a half: 4.7, 5.5).
 DecodeChoice choose_decode(int m, int n, int k, int l, int num_sms, const nvfp4_gemm_config& cf) {
     if (cf.cta_group == 2 || cf.tile_n != 0 || cf.grid != 0 || cf.split_k != 0 || cf.epilogue != 0) return DecodeChoice{0, 0, false};
     const int tokens = m <= 32 ? 32 : m <= 64 ? 64 : 128;
@@ -499,6 +506,8 @@ DecodeChoice choose_decode(int m, int n, int k, int l, int num_sms, const nvfp4_
     else if (tiles * 32 <= num_sms * 7LL && k_tiles >= (tiles * 8 <= num_sms ? (wide ? 12 : 8) : 24)) split = 4;
     else if (tiles * 2 <= num_sms && k_tiles >= (tiles * 4 <= num_sms ? 12 : wide ? 16 : 24)) split = 2;
     if (wide && split == 1) split = 0;
+    const bool many = tokens == 64 ? tiles > 2LL * num_sms : k_tiles < 4 && tiles > 4LL * num_sms;
+    if (split == 1 && many) split = 0;
     return DecodeChoice{tokens, split, split == 1 && tiles > num_sms};
 }
 

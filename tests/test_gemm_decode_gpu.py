@@ -43,6 +43,19 @@ def test_decode_matches_oracle_bit_exact(sub, oracle, shape, kernel):
         assert_bit_exact(data[6], exp, what=f"{shape} {sub.last_kernel()}")
 
 
+# many tiles per SM: where the persistent kernels take over
+@pytest.mark.parametrize("shape,decode", [((17, 25344, 512, 3), False), ((17, 25344, 1024, 3), True), ((50, 19072, 512, 2), False), ((50, 18944, 512, 2), True)])
+def test_many_tiles(sub, oracle, shape, decode):
+    from nvfp4_gemm_b200.inputs import generate_input
+    data = generate_input(*shape, 79)
+    data[6].view(torch.int16).fill_(0x7fff)
+    sub.custom_kernel(data)
+    sub.check_status()
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert ("decode" in sub.last_kernel()) == decode
+    assert_bit_exact(data[6], expected_fp16(oracle, data), what=f"{shape} {sub.last_kernel()}")
+
+
 @pytest.mark.parametrize("shape,kernel", CASES)
 def test_decode_epilogue_equals_the_persistent_kernels(sub, shape, kernel):
     """Bias, ReLU and re-quantising give the bytes that the 128-row-tile kernels give; rows of the last
