@@ -7,13 +7,13 @@
 // published as fp32 partials in per-worker scratch slots by all but the worker that holds the
 // start of its k-range, which sums the partials in a fixed order (deterministic) and writes fp16;
 // SegmentPlan orders a worker's pieces so that this summing runs beside later whole tiles.
-// Decode shapes (one 128-row block) split K over a cluster instead (KS > 1).
+// K may be split over a cluster instead (KS > 1, where the caller asks for it; few rows run gemm_decode_sm100.cuh).
 //
 // A worker is one CTA (CG = 1: 128 x BN tile) or a CTA pair running tcgen05 with cta_group::2
 // (CG = 2: 256 x BN tile; each CTA holds 128 rows of A, BN/2 rows of B and its own 128
 // accumulator rows, so B crosses L2 -> SM once per pair).
 //
-// Warp roles (320 threads per CTA; 192 in the cluster split-K kernels):
+// Warp roles (320 threads per CTA, or 192: see kEpiWarps):
 //   warp 0      TMA producer: A/B tiles (128-byte swizzle) and the 512-byte scale atoms of the
 //               permuted layout into a STAGES-deep shared-memory ring (full/empty mbarriers)
 //   warp 1      TMEM owner.  Leader CTA: MMA issuer, ONE thread elected once -- tcgen05.cp scale
@@ -114,9 +114,12 @@ struct GemmSmem {
     // Epilogue scratch: TMA-store staging (two 32-row x 128-byte buffers per warp), or the landing
     // area of the cluster split-K exchange.
     static constexpr uint32_t kEpiBytes = EPI_KB * 1024;
-    // Epilogue warps: two groups of four (each covers the 128 TMEM lanes) share a tile's columns; the
-    // cluster split-K kernels have one group.
-    static constexpr int kEpiWarps = KS == 1 ? 8 : 4;
+    // Epilogue warps: two groups of four (each covers the 128 TMEM lanes) share a tile's columns where the epilogue
+    // is what a launch waits for (128 x 7168 x 2048 on single CTAs: 5.6 -> 4.9 us; SiLU with re-quantising on pairs:
+    // 40 -> 29).  One group for the cluster split-K kernels and for 256-wide pair tiles stored by TMA, which gain
+    // nothing from a second one (1000 x 4096 x 4096: 11.13 us, with two 11.15; 4096 x 7168 x 7168: 96.3, 96.9).
+    static constexpr bool kWideTmaStore = CG == 2 && BN == 256 && TMA_STORE;
+    static constexpr int kEpiWarps = KS > 1 || kWideTmaStore ? 4 : 8;
     static constexpr int kThreads = 64 + 32 * kEpiWarps;
     static constexpr uint32_t kStagingBufs = TMA_STORE ? (EPI_KB * 1024 / kEpiWarps) / 4096 : 1;   // 32-row x 128-byte buffers per epilogue warp
     static constexpr uint32_t kStagingPerWarp = kStagingBufs * 32 * 128;
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
     constexpr int kGroups = S::kEpiWarps / 4;                          // epilogue warp groups
     constexpr int kMyRelease = kReleaseAfter / kGroups;                // pieces a group drains before the hand-back
     constexpr int kMyChunks = kChunks / kGroups;                       // pieces a group drains in all
+    static_assert(KS > 1 || ((kMyRelease == 2 || kMyRelease == 4) && kMyChunks % 2 == 0), "the hand-back follows the first 64 or 128 columns");
     constexpr int kSfbColsPerMma = BN / 32;  // 4 TMEM columns per 128 rows of B
     constexpr int kBRows = S::kBRows;
 
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
             ptx::mbar_init(bar_fix_full + b * 8, (KS > 1 && b == 0) ? (S::kBulkExchange ? 1 : 128 * (KS - 1)) : (KS > 1 && b == 1) ? (KS - 1) : 1);
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(bar_acc_full + a * 8, 1);
-            ptx::mbar_init(bar_acc_empty + a * 8, kEpiThreads * CG);
+            ptx::mbar_init(bar_acc_empty + a * 8, S::kEpiWarps * CG);
         }
         *abort_flag = 0u;
         ptx::fence_mbar_init();
@@ -671,10 +675,14 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                 }
             };
             auto release_acc = [&]() {
+                // (all lanes' loads are complete; one arrival per warp, half of them cross to the pair's leader)
                 ptx::tc_fence_before();
+                __syncwarp();
                 const uint32_t bar = bar_acc_empty + (kAccOverlap ? 0u : acc * 8);
-                if (CG == 2 && !leader) ptx::mbar_arrive_cluster_signal(bar, 0);
-                else ptx::mbar_arrive(bar);
+                if (lane == 0) {
+                    if (CG == 2 && !leader) ptx::mbar_arrive_cluster_signal(bar, 0);
+                    else ptx::mbar_arrive(bar);
+                }
             };
 
             if constexpr (KS > 1) {
@@ -907,13 +915,22 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                                           make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
                     };
+                    if constexpr (kMyRelease == 4) {
+                        uint32_t held[4][32];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) ptx::tc_ld_32cols(t_acc + my_chunk(i) * 32, held[i]);
+                        ptx::tc_wait_ld();
+                        release_acc();  // the MMA warp may start the next tile now
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) publish32(my_chunk(i) * 32, held[i]);
+                    }
 #pragma unroll 1
-                    for (int i = 0; i < kMyChunks; i += 2) {
+                    for (int i = kMyRelease == 4 ? 4 : 0; i < kMyChunks; i += 2) {
                         uint32_t va[32], vb[32];
                         ptx::tc_ld_32cols(t_acc + my_chunk(i) * 32, va);
                         ptx::tc_ld_32cols(t_acc + my_chunk(i + 1) * 32, vb);
                         ptx::tc_wait_ld();
-                        if (i == 0) release_acc();  // the MMA warp may start the next tile now
+                        if (kMyRelease == 2 && i == 0) release_acc();
                         publish32(my_chunk(i) * 32, va);
                         publish32(my_chunk(i + 1) * 32, vb);
                     }
@@ -932,39 +949,24 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                     // fetches it cold, line by line through L2.  (Unrolled over the tile and over the scale
                     // blocks of a step, the re-quantising form with SiLU took 17 us longer after another
                     // kernel than after itself.)  What the hand-back waits for is the first step's: it goes to
-                    // registers, the accumulator is released, and only then anything is waited for, converted or stored.
-                    static_assert(kMyRelease == 2 && kMyChunks % 2 == 0, "the hand-back follows the first 64 columns");
-                    bool ready = true;
-#pragma unroll 1
-                    for (int i = 0; i < kMyChunks; i += 2) {
-                        const int c0 = my_chunk(i) * 32;             // (my_chunk(i + 1) is the neighbour)
-                        float s[64];
-                        {
-                            uint32_t va[32], vb[32];
-                            ptx::tc_ld_32cols(t_acc + c0, va);
-                            ptx::tc_ld_32cols(t_acc + c0 + 32, vb);
-                            ptx::tc_wait_ld();
-#pragma unroll
-                            for (int e = 0; e < 32; ++e) { s[e] = __uint_as_float(va[e]); s[32 + e] = __uint_as_float(vb[e]); }
-                        }
-                        if (i == 0) {
-                            release_acc();
-                            if (!whole_tile) {
-                                if (epi_tid == 0) {
-                                    const long long t_spin = clock64();
-                                    while (ptx::ld_acquire_gpu(counter) < need) {
-                                        if (*abort_flag || static_cast<uint64_t>(clock64() - t_spin) > timeout) {
-                                            *abort_flag = 1u;
-                                            ready = false;
-                                            break;
-                                        }
-                                        __nanosleep(64);
-                                    }
+                    // registers, the accumulator is released, and only then anything is waited for, converted or
+                    // stored; one group of warps over 256 columns (plain stores of little code) holds two steps.
+                    auto wait_for_others = [&]() {
+                        bool ready = true;
+                        if (epi_tid == 0) {
+                            const long long t_spin = clock64();
+                            while (ptx::ld_acquire_gpu(counter) < need) {
+                                if (*abort_flag || static_cast<uint64_t>(clock64() - t_spin) > timeout) {
+                                    *abort_flag = 1u;
+                                    ready = false;
+                                    break;
                                 }
-                                ready = ptx::named_bar_and(1, kEpiThreads, ready);
-                                if (!ready) break;
+                                __nanosleep(64);
                             }
                         }
+                        return ptx::named_bar_and(1, kEpiThreads, ready);
+                    };
+                    auto finish64 = [&](int c0, float (&s)[64]) {       // own sums in, total out
 #pragma unroll 1
                         for (int w = w_first + 1; w <= w_last; ++w) {   // later contributors use their "head" slot
                             const float* src = p.scratch + static_cast<long long>(partial_slot(w, 1, CG, cta_rank)) * (kBM * BN) + row_in_tile * 4;
@@ -978,6 +980,41 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                         }
                         if (row < p.M) emit(c0, s);
                         __syncwarp();
+                    };
+                    bool ready = true;
+                    if constexpr (kMyRelease == 4) {
+                        uint32_t held[4][32];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) ptx::tc_ld_32cols(t_acc + my_chunk(i) * 32, held[i]);
+                        ptx::tc_wait_ld();
+                        release_acc();
+                        if (!whole_tile && !wait_for_others()) break;
+#pragma unroll
+                        for (int i = 0; i < 4; i += 2) {
+                            float s[64];
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) { s[e] = __uint_as_float(held[i][e]); s[32 + e] = __uint_as_float(held[i + 1][e]); }
+                            finish64(my_chunk(i) * 32, s);
+                        }
+                    }
+#pragma unroll 1
+                    for (int i = kMyRelease == 4 ? 4 : 0; i < kMyChunks; i += 2) {
+                        const int c0 = my_chunk(i) * 32;             // (my_chunk(i + 1) is the neighbour)
+                        float s[64];
+                        {
+                            uint32_t va[32], vb[32];
+                            ptx::tc_ld_32cols(t_acc + c0, va);
+                            ptx::tc_ld_32cols(t_acc + c0 + 32, vb);
+                            ptx::tc_wait_ld();
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) { s[e] = __uint_as_float(va[e]); s[32 + e] = __uint_as_float(vb[e]); }
+                        }
+                        if (kMyRelease == 2 && i == 0) {
+                            release_acc();
+                            if (!whole_tile) ready = wait_for_others();
+                            if (!ready) break;
+                        }
+                        finish64(c0, s);
                     }
                     if (!ready) break;
                     if (!whole_tile && epi_tid == 0) *counter = 0;
