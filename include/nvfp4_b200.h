@@ -61,7 +61,7 @@ typedef struct nvfp4_gemm_config {
     int32_t epilogue;  /* 0 auto, 1 = 16-byte global stores, 2 = TMA store, 3 = TMA store with four staging buffers per warp */
     int32_t grid;      /* 0 auto (one CTA per SM), else number of persistent CTAs */
     int32_t cta_group; /* 0 auto, 1 = one CTA per tile, 2 = CTA pair per 256-row tile */
-    int32_t split_k;   /* 0 auto, 1 = persistent stream-K kernel, 2, 4 or 8 = cluster split-K (reduce in DSMEM; 8 needs tile_n 256) */
+    int32_t split_k;   /* 0 auto (few rows: the decode kernel, which splits K by its own rule), 1 = persistent stream-K kernel, 2, 4 or 8 = cluster split-K with 128-row tiles (8 needs tile_n 256) */
     int32_t raster;    /* tile order of the persistent kernels: 0 auto, -1 = row-major, r > 0 = column-major inside groups of r row tiles */
 } nvfp4_gemm_config;
 
