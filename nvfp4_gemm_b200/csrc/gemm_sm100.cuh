@@ -115,7 +115,7 @@ struct GemmSmem {
     // area of the cluster split-K exchange.
     static constexpr uint32_t kEpiBytes = EPI_KB * 1024;
     // Epilogue warps: two groups of four (each covers the 128 TMEM lanes) share a tile's columns where the epilogue
-    // is what a launch waits for (128 x 7168 x 2048 on single CTAs: 5.6 -> 4.9 us; SiLU with re-quantising on pairs:
+    // is what a launch waits for (128 x 7168 x 2048 on single CTAs, operands in L2: 5.6 -> 4.9 us; SiLU with re-quantising on pairs:
     // 40 -> 29).  One group for the cluster split-K kernels and for 256-wide pair tiles stored by TMA, which gain
     // nothing from a second one (1000 x 4096 x 4096: 11.13 us, with two 11.15; 4096 x 7168 x 7168: 96.3, 96.9).
     static constexpr bool kWideTmaStore = CG == 2 && BN == 256 && TMA_STORE;
