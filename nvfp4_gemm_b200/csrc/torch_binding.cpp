@@ -129,16 +129,17 @@ nvfp4_problem make_problem(const Operands& o) {
 }
 
 // Calls f(stream) with the tensors' device current, on torch's current stream of that device and
-// without the interpreter lock (a launch waits when the queue of the device is full).
+// without the interpreter lock (a launch waits when the queue of the device is full).  Only f, which
+// answers with a status, runs unlocked: the guard and the stream throw where CUDA reports an error, and
+// an exception that left with the lock released would be turned into a Python one without a thread state.
 template <class F>
 int on_current_stream(const at::Tensor& a, F f) {
     const c10::DeviceIndex dev = a.device().index();
+    const c10::cuda::CUDAGuard guard(dev);
+    void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
     int rc = 0;
     Py_BEGIN_ALLOW_THREADS
-    {
-        const c10::cuda::CUDAGuard guard(dev);
-        rc = f(static_cast<void*>(c10::cuda::getCurrentCUDAStream(dev).stream()));
-    }
+    rc = f(stream);
     Py_END_ALLOW_THREADS
     return rc;
 }

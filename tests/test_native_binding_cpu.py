@@ -1,4 +1,8 @@
 """The native module's translation of the operator's 7-tuple: what it accepts and what it refuses."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -36,3 +40,32 @@ def test_entry_points_refuse_cpu_tensors(lib):
     for call in (custom_kernel, gemm_epilogue, lambda d: custom_kernel(list(d))):
         with pytest.raises(ValueError, match="no CPU fallback"):
             call(data)
+
+
+_ON_NO_DEVICE = """
+import torch
+from nvfp4_gemm_b200 import submission
+
+class Elsewhere(torch.Tensor):
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise AssertionError(func)
+
+def tensor(rows, cols, dtype):
+    return torch.Tensor._make_wrapper_subclass(Elsewhere, (rows, cols, 1), strides=(cols, 1, rows * cols), dtype=dtype, device="cuda:63")
+
+data = (tensor(128, 128, torch.uint8), tensor(256, 128, torch.uint8), None, None, None, None, tensor(128, 256, torch.float16))
+for call in (submission.custom_kernel, submission.gemm_epilogue):
+    try:
+        call(data)
+    except RuntimeError as e:
+        print("refused:", type(e).__name__)
+"""
+
+
+def test_a_cuda_error_ahead_of_the_call_is_a_python_exception(lib):
+    """Tensors that say they are on a device which no machine has: making it current fails, inside the
+    native module.  (In a process of its own: the failure to guard against is a crash.)"""
+    r = subprocess.run([sys.executable, "-c", _ON_NO_DEVICE], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.splitlines() == ["refused: RuntimeError"] * 2
