@@ -162,10 +162,12 @@ def native():
     if _native is None:
         load()
         import torch  # noqa: F401  (its libraries have to be in the process first)
-        try:
-            from . import _native as module
-        except ImportError as e:
-            raise ImportError(f"_native.so is missing or does not fit this torch ({e}): build it with `python -m nvfp4_gemm_b200.build`") from e
+        from . import build
+        built_for, target = build.binding_built_for(), build.binding_target()
+        if built_for != target:
+            raise ImportError(f"_native.so is {'built for ' + built_for if built_for else 'missing or out of date'}, this is {target}: "
+                              "build it with `python -m nvfp4_gemm_b200.build`")
+        from . import _native as module
         _native = module
     return _native
 

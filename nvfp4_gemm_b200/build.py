@@ -43,8 +43,27 @@ def _newer(target: Path, inputs: list[Path]) -> bool:
     return target.exists() and all(s.stat().st_mtime <= target.stat().st_mtime for s in inputs)
 
 
+def binding_target() -> str:
+    """What ``_native.so`` has to be built for: it holds layouts of torch's and Python's own types."""
+    import torch
+    return f"torch {torch.__version__}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, {sysconfig.get_config_var('SOABI')}"
+
+
+def binding_built_for() -> str | None:
+    """What the ``_native.so`` that is there was built for (the module carries it as a text)."""
+    if not BINDING.exists():
+        return None
+    mark = b"nvfp4_native built for: "
+    _, found, rest = BINDING.read_bytes().partition(mark)
+    return rest.partition(b"\0")[0].decode() if found else None
+
+
+def _binding_current() -> bool:
+    return _newer(BINDING, [BINDING_SRC, HEADER]) and binding_built_for() == binding_target()
+
+
 def needs_build() -> bool:
-    return not _newer(LIB, sources()) or not _newer(BINDING, [BINDING_SRC, HEADER])
+    return not _newer(LIB, sources()) or not _binding_current()
 
 
 def _replace(target: Path, cmd: list[str], verbose: bool) -> None:
@@ -64,7 +83,7 @@ def _build_binding(verbose: bool) -> None:
                 Path(sysconfig.get_paths()["include"])]
     # (torch's own libraries are in the process when the module is loaded: torch is imported first)
     _replace(BINDING, ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-                       f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                       f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DNVFP4_BUILT_FOR="{binding_target()}"',
                        *[f for i in includes for f in ("-isystem", str(i))], str(BINDING_SRC),
                        f"-L{PKG_DIR}", "-l:libnvfp4_b200.so", f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
                        "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], verbose)
@@ -73,7 +92,7 @@ def _build_binding(verbose: bool) -> None:
 def build(force: bool = False, verbose: bool = False) -> Path:
     if force or not _newer(LIB, sources()):
         _replace(LIB, [find_nvcc(), *(["-Xptxas", "-v"] if verbose else []), *NVCC_FLAGS, str(SRC)], verbose)
-    if force or not _newer(BINDING, [BINDING_SRC, HEADER]):
+    if force or not _binding_current():
         _build_binding(verbose)
     return LIB
 

@@ -229,6 +229,9 @@ PyObject* py_gemm_epilogue(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     });
 }
 
+// Read from the file by nvfp4_gemm_b200/build.py: the types of torch and Python that this code has the layouts of.
+[[gnu::used]] const char built_for[] = "nvfp4_native built for: " NVFP4_BUILT_FOR;
+
 PyMethodDef methods[] = {
     {"matmul", py_matmul, METH_O, "matmul(data) -> status"},
     {"fill_problem", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_fill_problem)), METH_FASTCALL, "fill_problem(data, address)"},
