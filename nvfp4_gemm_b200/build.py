@@ -1,8 +1,9 @@
 """Ahead-of-time build of the CUDA library and the torch binding (``python -m nvfp4_gemm_b200.build``).
 
 Compiles ``csrc/nvfp4_api.cu`` for sm_100a into ``libnvfp4_b200.so`` and ``csrc/torch_binding.cpp``
-(host code only) into ``_native.so`` next to this file.  nvcc cross-compiles without a GPU.  Nothing is JIT-compiled at call time (the reference
-builds at import with ``load_inline``, s_128t.py:587-602).
+(host code only) into ``_native.so`` next to this file.  nvcc cross-compiles without a GPU.  The first
+needs nvcc alone, the second g++ and the torch that it will run with.  Nothing is JIT-compiled at call
+time (the reference builds at import with ``load_inline``, s_128t.py:587-602).
 """
 from __future__ import annotations
 
@@ -58,12 +59,27 @@ def binding_built_for() -> str | None:
     return rest.partition(b"\0")[0].decode() if found else None
 
 
+def why_no_binding() -> str | None:
+    """The binding serves callers with torch; why it cannot be built here, or None."""
+    try:
+        import torch
+    except ImportError as e:
+        return f"torch cannot be imported ({e})"
+    if shutil.which("g++") is None:
+        return "g++ was not found"
+    if not (Path(torch.__file__).resolve().parent / "include" / "torch" / "csrc" / "autograd" / "python_variable.h").exists():
+        return "this torch has no headers"
+    if not (Path(sysconfig.get_paths()["include"]) / "Python.h").exists():
+        return "Python's headers are not installed"
+    return None
+
+
 def _binding_current() -> bool:
     return _newer(BINDING, [BINDING_SRC, HEADER]) and binding_built_for() == binding_target()
 
 
 def needs_build() -> bool:
-    return not _newer(LIB, sources()) or not _binding_current()
+    return not _newer(LIB, sources()) or (why_no_binding() is None and not _binding_current())
 
 
 def _replace(target: Path, cmd: list[str], verbose: bool) -> None:
@@ -90,9 +106,14 @@ def _build_binding(verbose: bool) -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
+    """Builds what is out of date.  The C library needs nvcc alone; where the binding cannot be built, a
+    caller of the C library is told so and gets it all the same (``_lib.native()`` refuses to go on without)."""
     if force or not _newer(LIB, sources()):
         _replace(LIB, [find_nvcc(), *(["-Xptxas", "-v"] if verbose else []), *NVCC_FLAGS, str(SRC)], verbose)
-    if force or not _binding_current():
+    why = why_no_binding()
+    if why is not None:
+        print(f"{BINDING.name} (calls on torch tensors) is not built: {why}", file=sys.stderr)
+    elif force or not _binding_current():
         _build_binding(verbose)
     return LIB
 

@@ -1,5 +1,6 @@
-"""What the build does where torch is another than before."""
+"""What the build does where torch, its headers or a compiler are not there, or are others than before."""
 import os
+import sys
 
 import pytest
 
@@ -23,6 +24,18 @@ def elsewhere(tmp_path, monkeypatch):
     monkeypatch.setattr(build, "BINDING", tmp_path / "_native.so")
     monkeypatch.setattr(build, "_replace", compile_)
     return asked
+
+
+@pytest.mark.parametrize("missing", ["torch", "g++"])
+def test_the_c_library_is_built_without_torch_or_a_host_compiler(elsewhere, monkeypatch, capsys, missing):
+    if missing == "torch":
+        monkeypatch.setitem(sys.modules, "torch", None)
+    else:
+        monkeypatch.setattr(build.shutil, "which", lambda name: None if name == "g++" else "/usr/bin/" + name)
+    monkeypatch.setattr(build, "find_nvcc", lambda: "nvcc")
+    assert build.build(force=True) == build.LIB
+    assert elsewhere == ["libnvfp4_b200.so"] and missing in capsys.readouterr().err
+    assert not build.needs_build()
 
 
 def test_a_binding_of_another_torch_is_built_again_and_not_loaded(elsewhere, monkeypatch):
