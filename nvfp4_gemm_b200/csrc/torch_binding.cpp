@@ -205,11 +205,15 @@ PyObject* py_gemm_epilogue(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         }
         e.activation = int_arg(args[2]);
         if (args[3] != Py_None) {
-            if (!PyTuple_Check(args[3]) && !PyList_Check(args[3])) raise(PyExc_TypeError, "out must be (packed, sf, sf_permuted)");
-            if (PySequence_Fast_GET_SIZE(args[3]) < 3) raise(PyExc_IndexError, "out must be (packed, sf, sf_permuted)");
+            struct Sequence {          // any sequence will do
+                PyObject* seq;
+                ~Sequence() { Py_XDECREF(seq); }
+            } const out{PySequence_Fast(args[3], "out must be (packed, sf, sf_permuted)")};
+            if (!out.seq) throw PythonError{};
+            if (PySequence_Fast_GET_SIZE(out.seq) < 3) raise(PyExc_IndexError, "out must be (packed, sf, sf_permuted)");
             void* ptr[3];
             for (int i = 0; i < 3; ++i) {
-                const at::Tensor* t = tensor_or_none(PySequence_Fast_GET_ITEM(args[3], i));
+                const at::Tensor* t = tensor_or_none(PySequence_Fast_GET_ITEM(out.seq, i));
                 if (!t) raise(PyExc_TypeError, "out must be (packed, sf, sf_permuted)");
                 ptr[i] = t->data_ptr();
             }

@@ -43,6 +43,7 @@ def test_entry_points_refuse_cpu_tensors(lib):
 
 
 _ON_NO_DEVICE = """
+from collections import UserList
 import torch
 from nvfp4_gemm_b200 import submission
 
@@ -61,11 +62,28 @@ for call in (submission.custom_kernel, submission.gemm_epilogue):
     except RuntimeError as e:
         print("refused:", type(e).__name__)
 """
+_OUT_IN_A_SEQUENCE = """
+out = UserList([tensor(128, 128, torch.uint8), tensor(128, 16, torch.uint8), tensor(128, 16, torch.uint8)])
+try:
+    submission.gemm_epilogue(data, nvfp4_out=True, out=out)
+except RuntimeError as e:
+    print("accepted")
+"""
+
+
+def _run(text):
+    return subprocess.run([sys.executable, "-c", text], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
 
 
 def test_a_cuda_error_ahead_of_the_call_is_a_python_exception(lib):
     """Tensors that say they are on a device which no machine has: making it current fails, inside the
     native module.  (In a process of its own: the failure to guard against is a crash.)"""
-    r = subprocess.run([sys.executable, "-c", _ON_NO_DEVICE], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
+    r = _run(_ON_NO_DEVICE)
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.splitlines() == ["refused: RuntimeError"] * 2
+
+
+def test_out_may_be_any_sequence(lib):
+    """The three tensors are taken from whatever sequence holds them; the call then fails at the device, not before."""
+    r = _run(_ON_NO_DEVICE + _OUT_IN_A_SEQUENCE)
+    assert r.returncode == 0 and r.stdout.splitlines()[-1] == "accepted", r.stderr[-2000:]
