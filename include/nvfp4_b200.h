@@ -364,7 +364,7 @@ uint64_t nvfp4_launch_count(void);
 /* Name of the kernel variant the last nvfp4_gemm / nvfp4_gemv call on this thread launched. */
 const char* nvfp4_last_kernel(void);
 
-/* Frees cached tensor maps and scratch memory on every device. */
+/* Frees scratch memory on every device and forgets what is known of it; a later call sets both up again. */
 void nvfp4_shutdown(void);
 
 const char* nvfp4_last_error(void);

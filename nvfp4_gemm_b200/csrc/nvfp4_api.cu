@@ -81,7 +81,7 @@ struct DeviceCtx {
     size_t scratch_bytes = 0;
     std::atomic<bool> scratch_ready{false};   // scratch and counters are allocated and cleared
     int max_pairs = -1;  // CTA pairs that can be co-resident (cluster occupancy), queried once
-    bool smem_attr_set[24] = {};
+    std::atomic<bool> smem_attr_set[52] = {};   // by kernel variant: 0..23 the tiled kernels, 24.. the decode kernels
 };
 
 std::mutex g_mutex;
@@ -356,13 +356,13 @@ int launch_gemm_splitk(DeviceCtx* c, int variant, GemmParams& params, cudaStream
 
 // Decode launch: one cluster of KS CTAs per 128 output columns.
 template <int BT, int STAGES, int KS>
-int launch_gemm_decode(const DeviceCtx* c, const GemmParams& params, bool epi, cudaStream_t stream, const char* name) {
+int launch_gemm_decode(DeviceCtx* c, int variant, const GemmParams& params, bool epi, cudaStream_t stream, const char* name) {
     using S = DecodeSmem<BT, STAGES, KS>;
     auto kernel = epi ? gemm_decode_kernel<BT, STAGES, KS, true> : gemm_decode_kernel<BT, STAGES, KS, false>;
-    static std::atomic<uint64_t> attr_set[2];   // bit per device (ordinals are below 64)
-    if (!(attr_set[epi].load() >> c->device & 1u)) {
+    std::atomic<bool>& attr_set = c->smem_attr_set[24 + 2 * variant + epi];   // (with the rest of what is known of the device: nvfp4_shutdown forgets it)
+    if (!attr_set) {
         CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamicBytes));
-        attr_set[epi].fetch_or(1ull << c->device);
+        attr_set = true;
     }
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
@@ -511,24 +511,24 @@ DecodeChoice choose_decode(int m, int n, int k, int l, int num_sms, const nvfp4_
     return DecodeChoice{tokens, split, split == 1 && tiles > num_sms};
 }
 
-int launch_gemm_decode(const DeviceCtx* c, const GemmParams& g, const DecodeChoice& d, bool epi, cudaStream_t stream) {
+int launch_gemm_decode(DeviceCtx* c, const GemmParams& g, const DecodeChoice& d, bool epi, cudaStream_t stream) {
     if (d.tokens == 32) {
-        if (d.split == 8) return launch_gemm_decode<32, 8, 8>(c, g, epi, stream, "gemm_splitk8_decode_t32");
-        if (d.split == 4) return launch_gemm_decode<32, 8, 4>(c, g, epi, stream, "gemm_splitk4_decode_t32");
-        if (d.split == 2) return launch_gemm_decode<32, 8, 2>(c, g, epi, stream, "gemm_splitk2_decode_t32");
-        if (d.two_per_sm) return launch_gemm_decode<32, 4, 1>(c, g, epi, stream, "gemm_decode_t32_s4");
-        return launch_gemm_decode<32, 8, 1>(c, g, epi, stream, "gemm_decode_t32_s8");
+        if (d.split == 8) return launch_gemm_decode<32, 8, 8>(c, 0, g, epi, stream, "gemm_splitk8_decode_t32");
+        if (d.split == 4) return launch_gemm_decode<32, 8, 4>(c, 1, g, epi, stream, "gemm_splitk4_decode_t32");
+        if (d.split == 2) return launch_gemm_decode<32, 8, 2>(c, 2, g, epi, stream, "gemm_splitk2_decode_t32");
+        if (d.two_per_sm) return launch_gemm_decode<32, 4, 1>(c, 3, g, epi, stream, "gemm_decode_t32_s4");
+        return launch_gemm_decode<32, 8, 1>(c, 4, g, epi, stream, "gemm_decode_t32_s8");
     }
     if (d.tokens == 64) {
-        if (d.split == 8) return launch_gemm_decode<64, 7, 8>(c, g, epi, stream, "gemm_splitk8_decode_t64");
-        if (d.split == 4) return launch_gemm_decode<64, 7, 4>(c, g, epi, stream, "gemm_splitk4_decode_t64");
-        if (d.split == 2) return launch_gemm_decode<64, 7, 2>(c, g, epi, stream, "gemm_splitk2_decode_t64");
-        if (d.two_per_sm) return launch_gemm_decode<64, 3, 1>(c, g, epi, stream, "gemm_decode_t64_s3");
-        return launch_gemm_decode<64, 7, 1>(c, g, epi, stream, "gemm_decode_t64_s7");
+        if (d.split == 8) return launch_gemm_decode<64, 7, 8>(c, 5, g, epi, stream, "gemm_splitk8_decode_t64");
+        if (d.split == 4) return launch_gemm_decode<64, 7, 4>(c, 6, g, epi, stream, "gemm_splitk4_decode_t64");
+        if (d.split == 2) return launch_gemm_decode<64, 7, 2>(c, 7, g, epi, stream, "gemm_splitk2_decode_t64");
+        if (d.two_per_sm) return launch_gemm_decode<64, 3, 1>(c, 8, g, epi, stream, "gemm_decode_t64_s3");
+        return launch_gemm_decode<64, 7, 1>(c, 9, g, epi, stream, "gemm_decode_t64_s7");
     }
-    if (d.split == 8) return launch_gemm_decode<128, 4, 8>(c, g, epi, stream, "gemm_splitk8_decode_t128");
-    if (d.split == 4) return launch_gemm_decode<128, 4, 4>(c, g, epi, stream, "gemm_splitk4_decode_t128");
-    return launch_gemm_decode<128, 5, 2>(c, g, epi, stream, "gemm_splitk2_decode_t128");
+    if (d.split == 8) return launch_gemm_decode<128, 4, 8>(c, 10, g, epi, stream, "gemm_splitk8_decode_t128");
+    if (d.split == 4) return launch_gemm_decode<128, 4, 4>(c, 11, g, epi, stream, "gemm_splitk4_decode_t128");
+    return launch_gemm_decode<128, 5, 2>(c, 12, g, epi, stream, "gemm_splitk2_decode_t128");
 }
 
 int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_epilogue* epi, void* const* c_peers, int n_peers,
