@@ -35,11 +35,6 @@ def _require_cuda(data: input_t) -> None:
         raise ValueError("custom_kernel needs CUDA tensors (there is no CPU fallback)")
 
 
-def _layout_key(t) -> tuple:
-    """Everything of a tensor that make_problem() reads: address, shape and strides (None-safe)."""
-    return (0, (), ()) if t is None else (t.data_ptr(), tuple(t.shape), tuple(t.stride()))
-
-
 def custom_kernel(data: input_t) -> output_t:
     status = _lib.native().matmul(data)
     if status:

@@ -195,7 +195,7 @@ def test_bench_roofline_arithmetic_matches_the_stated_work():
             assert shape["k"] % 64 == 0 and (shape["n"] == 1 or shape["n"] % 128 == 0)
 
 
-def test_problem_cache_key_covers_strides_and_none_scales():
+def test_problem_covers_strides_and_none_scales():
     """Same storage seen through two stride layouts gives two distinct problem structs, and a
     GEMV-only call may leave the permuted scale tensors out."""
     import torch
@@ -204,11 +204,15 @@ def test_problem_cache_key_covers_strides_and_none_scales():
     data = generate_input(64, 1, 512, 1, 3, device="cpu")
     p = S.make_problem(data[:4] + (None, None, data[6]))
     assert p.sfa_perm is None and p.sfb_perm is None and p.n == 1
-    store = torch.zeros(64 * 512, dtype=torch.uint8)
-    v1 = torch.as_strided(store, (32, 256, 1), (256, 1, 32 * 256))
-    v2 = torch.as_strided(store, (32, 256, 1), (512, 1, 32 * 512))
-    assert v1.data_ptr() == v2.data_ptr() and S._layout_key(v1) != S._layout_key(v2)
-    assert S._layout_key(None) == (0, (), ())
+    store = torch.zeros(2 * 64 * 512, dtype=torch.uint8)
+    b = torch.zeros((2, 1, 256), dtype=torch.uint8).permute(1, 2, 0)
+    seen = []
+    for row, batch in ((256, 32 * 256), (512, 32 * 512)):
+        v = torch.as_strided(store, (32, 256, 2), (row, 1, batch))
+        c = torch.as_strided(torch.zeros(2 * 32 * 8, dtype=torch.float16), (32, 1, 2), (row // 256, 1, 32 * row // 256))
+        p = S.make_problem((v, b, None, None, None, None, c))
+        seen.append((p.a, p.a_row_stride, p.a_batch_stride, p.c_row_stride, p.c_batch_stride))
+    assert seen == [(store.data_ptr(), 256, 32 * 256, 1, 32), (store.data_ptr(), 512, 32 * 512, 2, 64)]
 
 
 @pytest.mark.parametrize("raster", [0, 1, 8, 16])
