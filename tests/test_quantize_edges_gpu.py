@@ -57,3 +57,25 @@ def test_values_that_are_no_numbers(lib, dtype):
     assert nibbles[1, :4].tolist() == [0x7, 0xF, 0x7, 0x0]
     assert nibbles[2, :3].tolist() == [0xF, 0x9, 0x0]
     assert not nibbles[3].any()
+
+
+def test_back_to_back_launches_respect_stream_order(lib):
+    """The quantiser may start before the kernel ahead of it has ended: its input is rewritten in place right
+    before each launch, and its outputs are read right after."""
+    rows, k = 2048, 7168
+    g = torch.Generator(device="cuda").manual_seed(5)
+    inputs = [torch.randn((rows, k), generator=g, device="cuda", dtype=torch.bfloat16) * 2.0 ** i for i in range(3)]
+    exp = []
+    for x in inputs:
+        exp.append([t.clone() for t in _quantize(lib, x, k)])
+        torch.cuda.synchronize()
+    work = torch.empty_like(inputs[0])
+    outs = []
+    for _ in range(5):
+        for x in inputs:
+            work.copy_(x)
+            outs.append([t.clone() for t in _quantize(lib, work, k)])
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        for got, e in zip(o, exp[i % 3]):
+            assert torch.equal(got, e), i
