@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
                             const int q = token / S::kPieceTokens;                     // the rank that finalises them
                             const int c = (token % S::kPieceTokens) / S::kChunkTokens;
                             const int slot = ks_rank - (ks_rank > q ? 1 : 0);          // q keeps the foreign pieces in rank order
-                                                        if (q != ks_rank)
+                            if (q != ks_rank)
                                 ptx::bulk_copy_to_cluster(ptx::mapa_u32(smem_base + S::kLandOff + slot * S::kPieceBytes + c * S::kChunkBytes, q),
                                                           smem_base + token * (kBM * 4), S::kChunkBytes, ptx::mapa_u32(bar_land + c * 8, q));
                         }
@@ -309,24 +309,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) gemm_decode_kernel(const __
     if (!cluster_waited) ptx::cluster_wait();
     ptx::tc_fence_before();
     __syncthreads();
-    if (*abort_flag) {
-        // Some wait ran out.  Give copies still in flight time to land, then report.
-        __nanosleep(20000);
-        if (threadIdx.x == 0) {
-            *reinterpret_cast<volatile int*>(p.status) = kStatusWaitTimeout;
-            __threadfence_system();
-        }
-        __syncthreads();
-    }
-    if constexpr (KS > 1) {
-        // no CTA may retire (or free TMEM) while another can still write into its shared memory
-        ptx::cluster_arrive();
-        ptx::cluster_wait();
-    }
+    meet_cluster<KS>(abort_flag, tmem_slot + 4, p.status);
+    const bool gave_up = KS > 1 && *abort_flag;
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc<1>(tmem_base, kDecodeTmemCols);
     }
+    if constexpr (KS > 1) leave_cluster(gave_up);
 }
 
 }  // namespace nvfp4

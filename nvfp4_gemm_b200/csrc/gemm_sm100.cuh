@@ -276,6 +276,49 @@ __device__ __forceinline__ void bias_act16(const GemmParams& p, int gcol, float*
     }
 }
 
+// At the end of a CTA whose wait ran out: longer than a copy into shared memory that is on its way can take.
+__device__ __forceinline__ void let_copies_land() {
+    constexpr long long kCycles = 40000;          // 20 us at the highest clock; a copy takes one or two
+    const long long t0 = clock64();
+    do __nanosleep(1000);                         // (may return at once)
+    while (clock64() - t0 < kCycles);
+}
+
+// The end of a CTA, RANKS of which make a cluster, once its threads have met; TMEM may be freed after it.
+// A CTA whose wait ran out lets its own operand loads and MMAs finish (every thread stays for it) and reports.
+//
+// No CTA may retire while another can still write into its shared memory or read from it.  Where no wait ran out,
+// meeting the cluster is enough: a rank arrives after all that is sent to it has landed.  But a
+// rank that gave up has not waited for that, and a peer that did not give up may send to it until that
+// peer arrives.  So a rank that gave up tells all others before it arrives; after the meeting
+// everybody knows and nobody sends any more, and leave_cluster keeps all of them, and with them the shared memory, for
+// longer than a copy on its way can take.  (The branch on the flag stands behind the freeing of TMEM: ahead of it,
+// it cost each launch 0.03 to 0.09 us.  All threads meet again: warps must not leave ahead of a barrier of the cluster.)
+template <int RANKS>
+__device__ __forceinline__ void meet_cluster(volatile uint32_t* abort_flag, uint32_t abort_flag_addr, int* status) {
+    if (*abort_flag) {
+        let_copies_land();
+        if (threadIdx.x == 0) {
+            *reinterpret_cast<volatile int*>(status) = kStatusWaitTimeout;
+            __threadfence_system();
+            for (int r = 0; RANKS > 1 && r < RANKS; ++r) ptx::st_shared_cluster_u32(ptx::mapa_u32(abort_flag_addr, r), 1u);
+        }
+    }
+    __syncwarp();   // (no barrier of the CTA depends on the flag: a peer may set it between two warps' looks)
+    if constexpr (RANKS > 1) {
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+    }
+}
+// gave_up: the flag as it is after meet_cluster, the same in all CTAs then.
+__device__ __forceinline__ void leave_cluster(bool gave_up) {
+    if (gave_up) {
+        let_copies_land();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+    }
+}
+
 template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1, bool EPI_EX = false>
 __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS>::kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ GemmParams p) {
     static_assert(!(EPI_EX && TMA_STORE), "the extended epilogue writes with plain stores");
@@ -1031,26 +1074,13 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
     if (!cluster_waited) ptx::cluster_wait();  // the start-up cluster phase, for warps that had no reason to wait earlier
     ptx::tc_fence_before();
     __syncthreads();
-    if (*abort_flag) {
-        // Some wait ran out.  Give copies still in flight time to land in shared memory before
-        // the CTA retires, then report.
-        __nanosleep(20000);
-        if (threadIdx.x == 0) {
-            *reinterpret_cast<volatile int*>(p.status) = kStatusWaitTimeout;
-            __threadfence_system();
-        }
-        __syncthreads();
-    }
-    if constexpr (CG == 2 || KS > 1) {
-        // no CTA may retire (or free TMEM) while another can still issue pair-wide work or write
-        // into its shared memory
-        ptx::cluster_arrive();
-        ptx::cluster_wait();
-    }
+    meet_cluster<CG * KS>(abort_flag, tmem_slot + 4, p.status);   // (nor may a pair's CTA leave while the other can still issue work for both)
+    const bool gave_up = KS > 1 && *abort_flag;
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc<CG>(tmem_base, kTmemCols);
     }
+    if constexpr (KS > 1) leave_cluster(gave_up);
     if constexpr (CG == 2) {
         ptx::cluster_arrive();
         ptx::cluster_wait();

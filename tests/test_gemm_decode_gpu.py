@@ -95,3 +95,36 @@ def test_rows_beyond_a_tile_width_pick_the_next_width_on_batches(sub, oracle):
         assert "decode" in sub.last_kernel()
         assert_bit_exact(wide.contiguous(), expected_fp16(oracle, (a, b, sfa, sfb, sfa_perm, sfb_perm, c)), what=f"m {m}")
         assert int((store.view(torch.int16) == 0x7E01).sum()) == l * m * 24
+
+
+# a limit is looked at about every millisecond, so the launch has to last some: K is long
+@pytest.mark.parametrize("m,kernel", [(32, "gemm_splitk8_decode_t32"), (128, "gemm_splitk8_decode_t128")])
+def test_a_split_that_gives_up_reports_it_and_leaves_together(sub, lib, oracle, m, kernel):
+    """With a limit of a nanosecond the ranks' waits run out while operands are still streaming in.  The launch
+    ends, the host hears of it, and what runs next is right."""
+    from nvfp4_gemm_b200 import _lib
+    from nvfp4_gemm_b200.inputs import FP4_DTYPE, SF_DTYPE, generate_input
+    n, k = 128, 1 << 25
+    codes = lambda rows: torch.full((1, rows, k // 2), 0x02, dtype=torch.uint8, device="cuda").permute(1, 2, 0).view(FP4_DTYPE)  # noqa: E731
+    atoms = torch.full((1, 1, k // 64, 32, 4, 4), 0x08, dtype=torch.uint8, device="cuda").permute(3, 4, 1, 5, 2, 0).view(SF_DTYPE)
+    c = torch.empty((1, m, n), dtype=torch.float16, device="cuda").permute(1, 2, 0)
+    data = (codes(m), codes(n), None, None, atoms, atoms, c)
+    small = generate_input(m, 256, 12288, 1, 3)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        prev = lib.nvfp4_set_wait_timeout_ns(1)
+        try:
+            sub.custom_kernel(data)
+        finally:
+            lib.nvfp4_set_wait_timeout_ns(prev)
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert sub.last_kernel() == kernel
+        with pytest.raises(_lib.Nvfp4Error) as e:
+            sub.check_status()
+        assert e.value.code == _lib.NVFP4_ERR_DEVICE_TIMEOUT
+        sub.custom_kernel(small)
+        sub.check_status()
+        assert_bit_exact(small[6], expected_fp16(oracle, small), what="after a launch that gave up")
+    sub.custom_kernel(data)
+    sub.check_status()
+    assert torch.equal(c, torch.full_like(c, k // 2 * 2.0 ** -12))     # 1 * 1 and 0 * 0 in turn, scales 2^-6: exact
