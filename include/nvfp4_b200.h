@@ -327,6 +327,13 @@ int nvfp4_plan_units(int total_units, int grid, int cta, int* begin, int* end, i
 int nvfp4_plan_work_split(int64_t tiles, int k_tiles, int max_workers, int* workers, int* whole_tiles);
 
 /*
+ * The rows [*begin, *end) of all l batches' rows (batch after batch, m each) that row worker `worker` of
+ * the matrix-vector product takes, where its workers go on in steps of step_rows rows and `resident` of them run at
+ * once; *workers is their number (a worker beyond it takes no rows).
+ */
+int nvfp4_plan_gemv_rows(int m, int l, int step_rows, int resident, int worker, int* workers, int* begin, int* end);
+
+/*
  * Host-side view of the tile a GEMM of this shape gets on a device with num_sms SMs when the
  * caller fixes nothing (cluster split-K aside, which decode shapes take first): *cta_group = 2 for
  * 256-row tiles on CTA pairs or 1, *tile_n = 128 or 256.  Pairs with 256 x 256 tiles unless the

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_nvfp4_kernel(const GemvPara
 // chunks of the vector once and walks rows of the matrix, four at a time with the next four in flight.
 // The matrix is then all that is loaded and converted, where the form above converts the vector again for
 // every R rows.  The partial sums of k_warps warps meet in shared memory.  The grid is resident at once
-// and the rows of all batches are split evenly over it, so short rows neither pay a CTA each nor end
+// and the rows are split evenly over it (plan_gemv_split), so short rows neither pay a CTA each nor end
 // in a ragged wave, and the launch can overlap the end of the kernel before it in the stream: the first
 // rows are asked into L2 ahead of the dependency wait.
 // Bound by HBM.  Measured (us, graph replay over rotating inputs, the form above -> this one): 7168 x 2048 x 4
@@ -202,6 +202,40 @@ constexpr int kGemvRowsPerStep = 4;
 constexpr int kGemvSliceChunks = 32;
 constexpr int kGemvMaxKWarps = 8;
 constexpr int kGemvBatchRows = 512;    // rows of a worker between two meetings of its warps
+
+// How the rows of all batches go to the row workers: every `sharers` workers in turn take sharers * rows_each + rows_left
+// rows, the first rows_left of them one more than the others.
+struct GemvSplit {
+    int workers, sharers, rows_each, rows_left;
+    __host__ __device__ void rows_of(int worker, int total, int* begin, int* end) const {   // none for a worker beyond the last
+        int i = worker, first = 0;
+        if (sharers < workers) {
+            const int share = worker / sharers;
+            i -= share * sharers;
+            first = share * (sharers * rows_each + rows_left);
+        }
+        const int b = first + i * rows_each + (i < rows_left ? i : rows_left), e = b + rows_each + (i < rows_left ? 1 : 0);
+        *begin = b < total ? b : total;
+        *end = e < total ? e : total;
+    }
+};
+// m rows of each of l batches, in steps of step_rows, over `resident` workers that run at once.  Evenly shared, a
+// worker may cross into the next batch, loads another vector and begins a step anew.  Up to three steps that shows
+// (1 x 8192, 8 batches: 2 workers with four batches each 5.6 us, 8 workers 2.2; 100 x 1024 x 8: 3.4 and 2.3; 1000 x 2112 x 8:
+// 6.5 and 5.2), and where workers cross batch after batch; there each batch has workers of its own if that takes no more
+// steps.  With more steps the few that cross are lost among them, and the even share is as fast or faster (7168 x 2048 x 4:
+// 7.8 us, by batches 8.5).
+inline GemvSplit plan_gemv_split(int m, int l, int step_rows, int resident) {
+    auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
+    const long long rows = static_cast<long long>(m) * l;
+    const long long own = resident / l < 1 ? 1 : resident / l < ceil_div(m, step_rows) ? resident / l : ceil_div(m, step_rows);
+    const long long own_steps = ceil_div(ceil_div(m, own), step_rows) * ceil_div(own * l, resident);
+    const long long all = resident < ceil_div(rows, step_rows) ? resident : ceil_div(rows, step_rows);
+    const long long all_rows = ceil_div(rows, all), all_steps = ceil_div(all_rows, step_rows), crossings = ceil_div(all_rows, m);
+    if (l > 1 && own_steps <= all_steps + crossings && (all_steps <= 3 || crossings > 1))
+        return GemvSplit{static_cast<int>(own * l), static_cast<int>(own), static_cast<int>(m / own), static_cast<int>(m % own)};
+    return GemvSplit{static_cast<int>(all), static_cast<int>(all), static_cast<int>(rows / all), static_cast<int>(rows % all)};
+}
 
 // Sums of four values over LANES neighbouring lanes; lanes that are a multiple of LANES / 4 hold value
 // (lane % LANES) / (LANES / 4).
@@ -220,18 +254,18 @@ __device__ __forceinline__ float lanes_sum4(const float (&v)[4], int lane) {
 }
 
 template <int LANES>
-__global__ void __launch_bounds__(kGemvMaxKWarps * 32, 2) gemv_resident_kernel(const GemvParams p, int k_warps, int row_workers, int rows_each,
-                                                                               int rows_left) {
+__global__ void __launch_bounds__(kGemvMaxKWarps * 32, 2) gemv_resident_kernel(const GemvParams p, int k_warps, int row_workers, GemvSplit split) {
     __shared__ float part[kGemvMaxKWarps * kGemvBatchRows];   // [row worker][row][k warp]
     constexpr int R = kGemvRowsPerStep;
     constexpr int kSub = 32 / LANES;                          // groups of lanes that take R rows each in a step of their warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int worker_in_cta = warp / k_warps, k_warp = warp % k_warps;
-    // rows [row_begin, row_end) of all batches' rows: rows_each per worker, the first rows_left workers take one more
+    // rows [row_begin, row_end) of all batches' rows
     const int worker = static_cast<int>(blockIdx.x) * row_workers + worker_in_cta;
-    const int row_begin = worker * rows_each + min(worker, rows_left), row_end = row_begin + rows_each + (worker < rows_left ? 1 : 0);
-    const int batch_rows = k_warps > 1 ? kGemvBatchRows : rows_each + 1;
-    const int batches = (rows_each + batch_rows) / batch_rows;   // the same for every warp of the grid
+    int row_begin, row_end;
+    split.rows_of(worker, p.M * p.L, &row_begin, &row_end);
+    const int batch_rows = k_warps > 1 ? kGemvBatchRows : split.rows_each + 1;
+    const int batches = (split.rows_each + batch_rows) / batch_rows;   // the same for every warp of the grid
     const int chunks = p.K / 64;
     const int chunk_begin = k_warp * chunks / k_warps, chunk_end = (k_warp + 1) * chunks / k_warps;
     const int chunk = chunk_begin + lane % LANES;

@@ -3,6 +3,7 @@
 // steady-state path of nvfp4_gemm / nvfp4_gemv.
 #include "../../include/nvfp4_b200.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -793,24 +794,25 @@ int nvfp4_gemv_config(const nvfp4_problem* p, int rows_per_warp, int warps_per_c
 
     // The vector fits the registers of the warps that share a row.  Lanes per row: as many
     // as it has 64-element chunks, rounded up to 8, 16 or 32 (more lanes would idle: 28672 x 512 x 8 took 48.4 us
-    // with a warp per row and 15.3 with 8 lanes), and no more CTAs than have a whole step of rows to do
-    // (2000 x 1024 x 8: 4.8 -> 3.7 us).
+    // with a warp per row and 15.3 with 8 lanes).
     const long long rows_total = static_cast<long long>(p->m) * p->l;
     const int chunks = p->k / 64;
+    const int k_warps = (chunks + kGemvSliceChunks - 1) / kGemvSliceChunks;
+    DeviceCtx* c = nullptr;
+    if (int rc = get_ctx(&c)) return rc;
     // Between 8192 and 14336 five to seven warps share a row, which leaves lanes or warps of the SM idle: the other
     // kernel is as fast or faster there (9000 x 12288 x 3: 32.3 us against 35.3; x 10240: 28.3, 28.3; x 14400: 41.2, 40.3).
-    const int k_warps = (chunks + kGemvSliceChunks - 1) / kGemvSliceChunks;
+    // (A few rows of K 4160 to 8192 take longer here where launches follow each other in a graph, 1000 x 5120 3.33 us against
+    // 2.82, and shorter where they are issued one by one, 940 x 5120 x 3 3.9 us against 6.1: the launches overlap.)
     if (rows_per_warp == 0 && warps_per_cta == 0 && (k_warps <= 4 || k_warps == kGemvMaxKWarps) && rows_total < (1 << 30)) {
-        DeviceCtx* c = nullptr;
-        if (int rc = get_ctx(&c)) return rc;
         // 128 registers a thread let 16 warps share an SM.  Three warps or more per row make a CTA of their own, so that
-        // as many of the 16 as possible are used (28672 x 4992: 19.9 us on 12 warps, 18.2 on 15).
-        const int row_workers = k_warps <= 2 ? kGemvMaxKWarps / k_warps : 1;
-        const int ctas_per_sm = 16 / (k_warps * row_workers);
+        // as many of the 16 as possible are used (28672 x 4992: 19.9 us on 12 warps, 18.2 on 15).  Others share a CTA of eight
+        // warps, or of fewer where few workers can be spread over more SMs (1000 x 1024 x 3: 2.8 us, spread 2.3).
         const int lanes = chunks <= 8 ? 8 : chunks <= 16 ? 16 : 32;
-        const long long step_rows = static_cast<long long>(row_workers) * kGemvRowsPerStep * (32 / lanes);   // one step of a CTA
-        long long ctas = (rows_total + step_rows - 1) / step_rows;
-        if (ctas > static_cast<long long>(ctas_per_sm) * c->num_sms) ctas = static_cast<long long>(ctas_per_sm) * c->num_sms;
+        const GemvSplit split = plan_gemv_split(p->m, p->l, kGemvRowsPerStep * (32 / lanes), 16 / k_warps * c->num_sms);
+        int row_workers = k_warps > 2 ? 1 : kGemvMaxKWarps / k_warps;
+        if (split.workers <= 4 * c->num_sms) row_workers = std::min(row_workers, (split.workers + c->num_sms - 1) / c->num_sms);
+        const int ctas = (split.workers + row_workers - 1) / row_workers;
         cudaLaunchConfig_t cfg;
         std::memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
@@ -822,9 +824,7 @@ int nvfp4_gemv_config(const nvfp4_problem* p, int rows_per_warp, int warps_per_c
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         auto kernel = lanes == 8 ? gemv_resident_kernel<8> : lanes == 16 ? gemv_resident_kernel<16> : gemv_resident_kernel<32>;
-        const long long workers = ctas * row_workers;
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, g, k_warps, row_workers, static_cast<int>(rows_total / workers),
-                                    static_cast<int>(rows_total % workers)));
+        CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, g, k_warps, row_workers, split));
         g_launches.fetch_add(1);
         t_last_kernel = lanes == 8 ? "gemv_resident_8" : lanes == 16 ? "gemv_resident_16" : "gemv_resident_32";
         return NVFP4_OK;
@@ -1177,6 +1177,17 @@ int nvfp4_plan_work_split(int64_t tiles, int k_tiles, int max_workers, int* work
     const WorkSplit split = plan_work_split(tiles, k_tiles, max_workers);
     *workers = split.workers;
     *whole_tiles = split.whole_tiles ? 1 : 0;
+    return NVFP4_OK;
+}
+
+int nvfp4_plan_gemv_rows(int m, int l, int step_rows, int resident, int worker, int* workers, int* begin, int* end) {
+    if (m < 1 || l < 1 || l > 65535 || static_cast<long long>(m) * l >= (1 << 30) || step_rows < 1 || resident < 1 || worker < 0 || worker >= (1 << 20) ||
+        !workers || !begin || !end)
+        return fail(NVFP4_ERR_INVALID_ARGUMENT, "bad row-split query");
+    const GemvSplit split = plan_gemv_split(m, l, step_rows, resident);
+    *workers = split.workers;
+    *begin = *end = m * l;
+    if (worker < split.workers) split.rows_of(worker, m * l, begin, end);
     return NVFP4_OK;
 }
 

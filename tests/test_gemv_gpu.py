@@ -62,6 +62,21 @@ def test_gemv_resident_edges(sub, oracle, shape):
         assert_bit_exact(data[6], exp, what=f"gemv {shape}")
 
 
+# rows of batches: workers of their own for each batch, left over in the last CTA, more batches than workers, rows shared
+# over batches because there are too many for workers of their own and too few for one each, many steps
+@pytest.mark.parametrize("shape", [(1, 8192, 8), (1, 2112, 8), (1, 64, 33), (10, 512, 32), (3, 16384, 3), (100, 1024, 8), (1000, 2112, 8), (5, 4096, 700), (1, 256, 5000),
+                                   (31, 640, 1500), (2, 14400, 400), (6000, 1088, 5)])
+def test_gemv_rows_of_batches(sub, oracle, shape):
+    from nvfp4_gemm_b200.inputs import generate_input
+    m, k, l = shape
+    data = generate_input(m, 1, k, l, 13)
+    data[6].view(torch.int16).fill_(0x7fff)
+    sub.custom_kernel(data)
+    torch.cuda.synchronize()
+    assert sub.last_kernel().startswith("gemv_resident")
+    assert_bit_exact(data[6], expected_fp16(oracle, data), what=f"gemv {shape} {sub.last_kernel()}")
+
+
 def test_gemv_back_to_back_launches_respect_stream_order(sub, lib):
     """The matrix-vector product may start before the kernel ahead of it has ended; its operands are
     rewritten in place right before each launch."""

@@ -229,3 +229,27 @@ def test_tile_order_visits_every_output_tile_once(lib, tiles_m, tiles_n, batches
         seen.add((b.value, r.value, c.value))
     assert len(seen) == tiles
     assert lib.nvfp4_plan_tile(tiles * k_tiles, workers, k_tiles, tiles_m, tiles_n, raster, tiles, ctypes.byref(b), ctypes.byref(r), ctypes.byref(c)) != 0
+
+
+@pytest.mark.parametrize("resident", [16 * 148, 5 * 148, 2 * 148])
+@pytest.mark.parametrize("step_rows", [4, 16])
+@pytest.mark.parametrize("m,l", [(1, 1), (1, 8), (1, 33), (10, 32), (100, 8), (1000, 8), (7168, 4), (40000, 4), (5, 700), (31, 1500), (1, 65535), (3, 4000)])
+def test_gemv_row_split(lib, m, l, step_rows, resident):
+    """Every row is taken once, in order; and workers have rows of two batches only where they have many."""
+    workers, begin, end = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+    plan = lambda w: lib.nvfp4_plan_gemv_rows(m, l, step_rows, resident, w, ctypes.byref(workers), ctypes.byref(begin), ctypes.byref(end))  # noqa: E731
+    assert plan(0) == 0 and workers.value >= 1
+    at, most, crossing = 0, 0, 0
+    for w in range(workers.value):
+        assert plan(w) == 0 and begin.value == at and end.value >= at
+        most = max(most, end.value - begin.value)
+        crossing += end.value > begin.value and begin.value // m != (end.value - 1) // m
+        at = end.value
+    assert at == m * l
+    assert plan(workers.value) == 0 and begin.value == end.value == m * l
+    own = max(1, min(resident // l, -(-m // step_rows)))
+    if crossing:            # only where that is few of many steps
+        assert most > 3 * step_rows
+    else:
+        assert most <= -(-m // own) or l == 1
+    assert lib.nvfp4_plan_gemv_rows(0, l, step_rows, resident, 0, ctypes.byref(workers), ctypes.byref(begin), ctypes.byref(end)) == _lib.NVFP4_ERR_INVALID_ARGUMENT
