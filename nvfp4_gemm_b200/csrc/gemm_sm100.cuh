@@ -103,7 +103,7 @@ constexpr int kPrefetchStages = 2;                  // stages of a CTA's first s
 constexpr int kGlobalExchangeMinSplit = 4;         // cluster split-K: from this split on the partial sums travel through L2
 constexpr int kScratchSlotFloats = kBM * 256;      // one partial-tile slot of the library's scratch (128 x 256 fp32)
 
-template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1>
+template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1, int EPI_WARPS = 0>
 struct GemmSmem {
     static constexpr uint32_t kBRows = BN / CG;
     static constexpr uint32_t kABytes = kBM * kBKBytes;
@@ -115,11 +115,14 @@ struct GemmSmem {
     // area of the cluster split-K exchange.
     static constexpr uint32_t kEpiBytes = EPI_KB * 1024;
     // Epilogue warps: two groups of four (each covers the 128 TMEM lanes) share a tile's columns where the epilogue
-    // is what a launch waits for (128 x 7168 x 2048 on single CTAs, operands in L2: 5.6 -> 4.9 us; SiLU with re-quantising on pairs:
-    // 40 -> 29).  One group for the cluster split-K kernels and for 256-wide pair tiles stored by TMA, which gain
-    // nothing from a second one (1000 x 4096 x 4096: 11.13 us, with two 11.15; 4096 x 7168 x 7168: 96.3, 96.9).
-    static constexpr bool kWideTmaStore = CG == 2 && BN == 256 && TMA_STORE;
-    static constexpr int kEpiWarps = KS > 1 || kWideTmaStore ? 4 : 8;
+    // is what a launch waits for (SiLU with re-quantising on pairs: 40 -> 29 us).  One group for the cluster split-K
+    // kernels and for those stored by TMA that gain nothing from a second one: 256-wide pair tiles (1000 x 4096 x 4096:
+    // 11.13 us, with two 11.15; 4096 x 7168 x 7168: 96.3, 96.9) and 128-wide tiles of single CTAs, where 128 more threads
+    // to start cost more than they save (128 x 4096 x 256, 4 batches: 4.09 us, with two 4.30; 512 x 4608 x 1024: 4.87,
+    // 5.12; over 185 shapes of up to two waves with K 256 to 7168 4.9 to 0.6 %) -- except over many tiles of one k-tile,
+    // which are all epilogue (EPI_WARPS = 8: 1000 x 4608 x 256 x 4 20.6 us, with one group 21.7).
+    static constexpr bool kOneGroup = TMA_STORE && ((CG == 2 && BN == 256) || (CG == 1 && BN == 128));
+    static constexpr int kEpiWarps = EPI_WARPS ? EPI_WARPS : KS > 1 || kOneGroup ? 4 : 8;
     static constexpr int kThreads = 64 + 32 * kEpiWarps;
     static constexpr uint32_t kStagingBufs = TMA_STORE ? (EPI_KB * 1024 / kEpiWarps) / 4096 : 1;   // 32-row x 128-byte buffers per epilogue warp
     static constexpr uint32_t kStagingPerWarp = kStagingBufs * 32 * 128;
@@ -319,10 +322,10 @@ __device__ __forceinline__ void leave_cluster(bool gave_up) {
     }
 }
 
-template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1, bool EPI_EX = false>
-__global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS>::kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ GemmParams p) {
+template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, int KS = 1, bool EPI_EX = false, int EPI_WARPS = 0>
+__global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS, EPI_WARPS>::kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ GemmParams p) {
     static_assert(!(EPI_EX && TMA_STORE), "the extended epilogue writes with plain stores");
-    using S = GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS>;
+    using S = GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS, EPI_WARPS>;
     constexpr int kNumAcc = S::kNumAcc;
     constexpr bool kAccOverlap = S::kAccOverlap;
     constexpr int kSfaCol = kAccOverlap ? kSfaColOverlap : kSfaColPlain;

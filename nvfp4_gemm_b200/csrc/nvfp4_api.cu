@@ -260,10 +260,10 @@ WorkSplit plan_work_split(long long tiles, int k_tiles, int max_workers) {
     return WorkSplit{cost_split, max_workers, false};
 }
 
-template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, bool EPI_EX = false>
+template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, bool EPI_EX = false, int EPI_WARPS = 0>
 int launch_gemm(DeviceCtx* c, int variant, GemmParams& params, int grid_request, cudaStream_t stream, const char* name) {
-    using S = GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB>;
-    auto kernel = gemm_nvfp4_kernel<CG, BN, STAGES, TMA_STORE, EPI_KB, 1, EPI_EX>;
+    using S = GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, 1, EPI_WARPS>;
+    auto kernel = gemm_nvfp4_kernel<CG, BN, STAGES, TMA_STORE, EPI_KB, 1, EPI_EX, EPI_WARPS>;
     if (!c->smem_attr_set[variant]) {
         CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamicBytes));
         c->smem_attr_set[variant] = true;
@@ -716,6 +716,9 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
         if (epilogue >= 2) return launch_gemm<2, 128, 6, true, 32>(c, 6, g, grid, stream, "gemm_2cta_n128_s6_tmastore");
         return launch_gemm<2, 128, 6, false, 32>(c, 7, g, grid, stream, "gemm_2cta_n128_s6_direct");
     }
+    // (eight epilogue warps for many tiles of one k-tile: see GemmSmem)
+    if (bn == 128 && epilogue >= 2 && g.k_tiles == 1 && g.total_units > 2 * c->num_sms)
+        return launch_gemm<1, 128, 5, true, 32, false, 8>(c, 21, g, grid, stream, "gemm_1cta_n128_s5_tmastore");
     if (bn == 128 && epilogue >= 2) return launch_gemm<1, 128, 5, true, 32>(c, 0, g, grid, stream, "gemm_1cta_n128_s5_tmastore");
     if (bn == 128) return launch_gemm<1, 128, 4, false, 64>(c, 1, g, grid, stream, "gemm_1cta_n128_s4_direct");
     if (epilogue >= 2) return launch_gemm<1, 256, 3, true, 32>(c, 2, g, grid, stream, "gemm_1cta_n256_s3_tmastore");
