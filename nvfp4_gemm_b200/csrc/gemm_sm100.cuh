@@ -1077,8 +1077,28 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
     if (!cluster_waited) ptx::cluster_wait();  // the start-up cluster phase, for warps that had no reason to wait earlier
     ptx::tc_fence_before();
     __syncthreads();
-    meet_cluster<CG * KS>(abort_flag, tmem_slot + 4, p.status);   // (nor may a pair's CTA leave while the other can still issue work for both)
-    const bool gave_up = KS > 1 && *abort_flag;
+    bool gave_up = false;
+    if constexpr (KS > 1) {
+        meet_cluster<KS>(abort_flag, tmem_slot + 4, p.status);
+        gave_up = *abort_flag;
+    } else {
+        // (kept apart from the above: the larger code cost the re-quantising kernels 1.5 to 3 %)
+        if (*abort_flag) {
+            // Some wait ran out.  Give copies still in flight time to land in shared memory before
+            // the CTA retires, then report.
+            __nanosleep(20000);
+            if (threadIdx.x == 0) {
+                *reinterpret_cast<volatile int*>(p.status) = kStatusWaitTimeout;
+                __threadfence_system();
+            }
+            __syncthreads();
+        }
+        if constexpr (CG == 2) {
+            // no CTA may retire (or free TMEM) while the other can still issue pair-wide work
+            ptx::cluster_arrive();
+            ptx::cluster_wait();
+        }
+    }
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc<CG>(tmem_base, kTmemCols);
