@@ -1,4 +1,4 @@
-// NVFP4 GEMM for few rows of activations (decode; up to 128, a few times 128 with K split):  C[M,N] (fp16) = (A x SFA) . (B x SFB)^T.
+// NVFP4 GEMM for few rows of activations (decode; up to 128, more with K split):  C[M,N] (fp16) = (A x SFA) . (B x SFB)^T.
 //
 // Operands are swapped on the tensor core: the weights B are the M operand (128 of their rows = output
 // columns per CTA), the activations A the N operand, BT = 32, 64 or 128 of them.  D[column, token]
@@ -8,11 +8,11 @@
 // are in flight, and what an SM can take in is 65 bytes a cycle (its TMA unit).  As the M
 // operand the activations took 16 KB of every 36 KB stage whatever the batch (128-row tile,
 // zero-filled beyond M); as the N operand they take 128 bytes a row of a batch rounded up to 32, so
-// that the ring holds more stages, and MMAs and epilogue shrink with the batch.  Measured (us, graph
-// replay over rotating inputs, the 128-row-tile kernels -> this one): 17 x 7168 x 2048 5.6 -> 4.1,
-// 17 x 7168 x 16384 15.1 -> 12.2 (5.5 TB/s), 8 x 28672 x 4096 20 -> 12.2, 50 x 4096 x 7168 9.1 -> 6.5,
-// 128 x 7168 x 16384 15.6 -> 14.5, 128 x 4096 x 7168 9.35 -> 8.1.  For 65 to 128 rows without a split the
-// 128-row-tile kernels stay ahead (128 x 28672 x 4096: 14.6 against 17.3).
+// that the ring holds more stages, and MMAs and epilogue shrink with the batch.  Measured (us, replays of 24
+// launches over rotating inputs beyond L2, both kernels in turn in one process; the 128-row-tile kernels -> this one):
+// 17 x 7168 x 2048 5.8 -> 4.2, 17 x 7168 x 16384 15.3 -> 12.5 (5.3 TB/s), 1 x 28672 x 4096 20.6 -> 13.0, 40 x 4096 x 7168
+// 9.1 -> 6.6, 128 x 7168 x 16384 15.9 -> 14.9 (replays of 200: 16.7 -> 15.2-15.6), 128 x 4096 x 7168 9.3 -> 8.0.  For 65 to 128
+// rows without a split the 128-row-tile kernels stay ahead (128 x 28672 x 4096: 14.6 against 17.3).
 //
 // K is split over the KS ranks of a cluster, so that there are enough CTAs to pull at HBM's rate.
 // Rank r finalises tokens [r, r + 1) * BT / KS of the tile.  The accumulator is turned round in
@@ -22,10 +22,10 @@
 // the sums overlap.  The landing area is not part of the operand ring: a rank may send as soon as it
 // is done, without asking whether its peers are.  The older exchange took K = 4096 to 9.1-10.1 us on
 // 7168 columns; this one 5.8 (17 rows) and 7.4 (128).
-// Tried and not kept: CTA pairs that halve the activations' bytes again (15.1 us where one CTA takes
-// 14.5: the ring is not what binds, and the pair meets before its first load); prefetching weights
-// into L2 further ahead than the ring (17.9 us: the TMA unit serves prefetches like loads); eight
-// epilogue warps (14.9 us).
+// Tried and not kept, on 128 x 7168 x 16384, each against this kernel in the same session: CTA pairs that halve the
+// activations' bytes again (15.1 us, this one 14.5-15.2: the ring is not what binds, and the pair meets before its
+// first load); prefetching weights into L2 further ahead than the ring (17.9, 15.1: the TMA unit serves prefetches
+// like loads); eight epilogue warps (14.9, 14.5).
 //
 // Warp roles as in gemm_sm100.cuh: warp 0 TMA producer, warp 1 MMA issuer, one thread each; warps
 // 2..5 epilogue.  Every wait is bounded.  No load uses cluster multicast.

@@ -111,7 +111,7 @@ struct GemmSmem {
     static constexpr uint32_t kSfaBytes = kMmaPerStage * kSfAtomBytes;
     static constexpr uint32_t kSfbBytes = (BN / 128) * kMmaPerStage * kSfAtomBytes;
     static constexpr uint32_t kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
-    // Epilogue scratch: TMA-store staging (two 32-row x 128-byte buffers per warp), or the landing
+    // Epilogue scratch: TMA-store staging (kStagingBufs 32-row x 128-byte buffers per warp), or the landing
     // area of the cluster split-K exchange.
     static constexpr uint32_t kEpiBytes = EPI_KB * 1024;
     // Epilogue warps: two groups of four (each covers the 128 TMEM lanes) share a tile's columns where the epilogue
@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
                     uint8_t* staging_gen = smem_gen + S::kEpiOff + (warp - 2) * S::kStagingPerWarp;
                     const uint32_t staging = smem_base + S::kEpiOff + (warp - 2) * S::kStagingPerWarp;
                     // Phase 1, drain: this thread's share of its accumulator row goes TMEM -> registers
-                    // -> fp16 pairs (BN/4 registers), the loads of the next 32 columns in flight while
+                    // -> fp16 pairs (half a register a column), the loads of the next 32 columns in flight while
                     // the previous ones are converted.  The accumulator is handed back to the MMA warp
                     // as soon as the last column is in registers, before anything is stored: the TMA
                     // stores queue behind the producer's loads in the same TMA unit and are slow to

@@ -177,9 +177,10 @@ int scratch_set_for(DeviceCtx* c, cudaStream_t stream, int* set) {
                 kStreamSets, c->device);
 }
 
-// Encodes a tensor map into caller storage.  Every call encodes its four or five maps anew, like the
-// reference (s_128t.py:569-577): one takes the CPU 49 ns, less than finding it in a table of a few
-// hundred under a lock, and a caller whose buffers are new pays no more.
+// Encodes a tensor map into caller storage.  Every call encodes its maps anew, like the reference
+// (s_128t.py:569-577): four or five, and where the decode kernel runs three of them a second time with its own boxes.
+// One takes the CPU 49 ns, less than finding it in a table of a few hundred under a lock, and a caller whose buffers are
+// new pays no more.
 int encode_map(const MapKey& key, CUtensorMap* out) {
     EncodeTiledFn encode = nullptr;
     if (int rc = find_encode(&encode)) return rc;
@@ -489,7 +490,10 @@ struct DecodeChoice {
 // More than 64 rows run here only when K is split (unsplit the 128-row-tile kernel is as fast or faster), so
 // two pays earlier: from K = 4096 on a whole wave (128 x 7168 x 4096: 7.38, 7.73 unsplit), and four from 3072.
 // More than 128 rows are several token tiles of 128, under the same rules: 256 x 1536 x 16384 takes 8.9 us (unsplit
-// 128 x 128 tiles 16.2, shared tiles 22.7), 256 x 4096 x 7168 8.2 (9.6), 384 x 1536 x 7168 6.8 (8.2).
+// 128 x 128 tiles 16.2, shared tiles 22.7), 256 x 4096 x 7168 8.2 (9.6), 384 x 1536 x 7168 6.8 (8.2), and so up to
+// 8192 rows, where few columns leave as few tiles (8192 x 128 x 7168: 10.8, 11.9; 4096 x 256 x 16384: 14.4, 19.3).  At K = 4096
+// a whole wave is even (2048 x 512: 6.7, 6.4; 200 x 2560: 6.25, 6.43) but with the extended epilogue far ahead (300 x 512 x 4
+// batches to NVFP4: 8.7, 20.9).
 // More tiles than SMs: two CTAs per SM, so that one's start and end hide behind the other
 // (17 x 28672 x 2048: 7.07 against 9.29 us); up to one wave the deep ring is ahead (12288 columns: 4.55, 5.07).
 // With many tiles per SM the persistent kernels, which overlap one tile's stores with the next one's
