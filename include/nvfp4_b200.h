@@ -321,8 +321,8 @@ int nvfp4_plan_units(int total_units, int grid, int cta, int* begin, int* end, i
  * is split at tile boundaries only), or *whole_tiles = 0 and *workers = max_workers (an even split
  * of all (tile, k-tile) units; tiles shared between workers are summed through scratch).  The choice
  * is the smaller of two estimates in k-tiles of run time: waves x k_tiles, and units / workers plus
- * 3 (a worker has two tiles' worth of units or more: the summing hides behind whole tiles) or 12 per
- * worker that shares a tile (at least 24).
+ * 16 (a worker has two tiles' worth of units or more: the summing hides in part behind whole tiles) or 12
+ * per worker that shares a tile (at least 24).
  */
 int nvfp4_plan_work_split(int64_t tiles, int k_tiles, int max_workers, int* workers, int* whole_tiles);
 

@@ -96,7 +96,8 @@ struct GemmParams {
     int tiles_m, tiles_n, k_tiles;  // tiles of (128*CG) x BN; k_tiles = K / 256
     int raster_rows;                // row tiles per group of the persistent kernels' tile order; 0 = row-major
     int total_units;                // tiles_m * tiles_n * L * k_tiles
-    int whole_tiles;                // 1: workers split the work at tile boundaries only (no tile is shared); raster_rows must be 0
+    int whole_tiles;                // 1: workers split the work at tile boundaries only (no tile is shared)
+    int order_k, order_total;           // units of a tile and of all tiles as the order of tiles counts them (tile_coords)
 };
 
 constexpr int kPrefetchStages = 2;                  // stages of a CTA's first segment prefetched into L2 ahead of the dependency wait
@@ -208,7 +209,8 @@ struct SegmentPlan {
 // ranks fill the output column by column inside groups of raster_rows row tiles -- a wave of
 // workers shares a few row blocks of A and a few column tiles of B through L2 instead of every
 // worker streaming its own pair from DRAM.
-// raster_rows = 0 keeps the plain row-major order of the linear tile index.
+// raster_rows = 0 keeps the plain row-major order of the linear tile index.  Where workers take whole tiles the
+// ranges are counted in tiles: k_tiles = 1, total_units = tiles.
 struct TileCoord {
     int l, mt, nt;
 };
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
     const SegmentPlan plan(u_begin, u_end, KT);   // (a cluster split-K CTA has one segment: its share of the tile's k-range)
     Segment first_seg{0, 0, 0};
     plan.at(0, &first_seg);
-    const TileCoord first_tc = tile_coords(first_seg.tile, n_workers, KT, p.total_units, p.tiles_m, p.tiles_n, (KS > 1) ? 0 : p.raster_rows);
+    const TileCoord first_tc = tile_coords(first_seg.tile, n_workers, p.order_k, p.order_total, p.tiles_m, p.tiles_n, (KS > 1) ? 0 : p.raster_rows);
     // The operands of this CTA's first two stages are asked into L2 now, ahead of the dependency wait:
     // a CTA of a back-to-back launch reaches this point while slower CTAs of the previous launch
     // are still running, and its first loads then find their lines in L2 instead of paying the
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
             const int tile = seg.tile;
             const int k0 = seg.u0 - tile * KT;
             const int k1 = k0 + (seg.u1 - seg.u0);
-            const TileCoord tc = (si == 0) ? first_tc : tile_coords(tile, n_workers, KT, p.total_units, p.tiles_m, p.tiles_n, (KS > 1) ? 0 : p.raster_rows);
+            const TileCoord tc = (si == 0) ? first_tc : tile_coords(tile, n_workers, p.order_k, p.order_total, p.tiles_m, p.tiles_n, (KS > 1) ? 0 : p.raster_rows);
             const int nb = tc.nt;
             const int mb = tc.mt * CG + cta_rank;  // 128-row block of this CTA
             const int l = tc.l;
@@ -617,7 +619,7 @@ __global__ void __launch_bounds__(GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, KS
             const int tile = seg.tile;
             const int k0 = seg.u0 - tile * KT;
             const int k1 = k0 + (seg.u1 - seg.u0);
-            const TileCoord tc = (si == 0) ? first_tc : tile_coords(tile, n_workers, KT, p.total_units, p.tiles_m, p.tiles_n, (KS > 1) ? 0 : p.raster_rows);
+            const TileCoord tc = (si == 0) ? first_tc : tile_coords(tile, n_workers, p.order_k, p.order_total, p.tiles_m, p.tiles_n, (KS > 1) ? 0 : p.raster_rows);
             const int nb = tc.nt;
             const int mb = tc.mt * CG + cta_rank;
             const int l = tc.l;

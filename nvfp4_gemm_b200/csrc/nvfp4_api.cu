@@ -237,32 +237,34 @@ bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) %
 
 // Whole tiles per worker, or an even split of all (tile, k-tile) units with shared tiles summed
 // through scratch?  In k-tiles of run time: whole tiles cost waves x k_tiles; the even split costs
-// units / workers plus the summing, which hides in part behind later whole tiles when a worker has at
-// least two tiles' worth of units (measured as 13 to 18 k-tiles on ten shapes with 192 to 320 tiles of 256 x 256 and
-// K 2048 to 8192, whole tiles against the split: 4096 x 4096 x 2048 20.8 us against 26.9, 3072 x 4096 x 4096
-// 24.1 against 27.2, 2048 x 7168 x 7168 49.8 against 44.9; counted as 16) and otherwise ends the launch
-// (publish, wait, read back:
+// units / workers plus the summing.  That hides in part behind later whole tiles when a worker has at
+// least two tiles' worth of units: measured as 13 to 18 k-tiles of the 256-wide pair kernel on ten shapes with 192 to
+// 320 tiles and K 2048 to 8192 (whole tiles against the split: 4096 x 4096 x 2048 20.8 us against 26.9, 3072 x 4096 x 4096
+// 24.1 against 27.2, 2048 x 7168 x 7168 49.8 against 44.9) and counted as 16, also for single CTAs (2048 x 2560 x 1024: 9.7 us
+// whole, 16.5 split; 64 x 28672 x 2048 x 4: 25.8, 28.6).  Otherwise it ends the launch (publish, wait, read back:
 // measured about as long as 24 k-tiles of the 256-wide pair kernel with two workers per tile --
 // 768 x 4096 x 4096 took 19.5 us split 74 ways and 10.6 us as 48 whole tiles -- and counted as 12
 // k-tiles per worker that shares a tile).
+constexpr double kSumming = 16.0;
 struct WorkSplit {
     double cost;        // k-tiles of run time
     int workers;
     bool whole_tiles;
 };
-WorkSplit plan_work_split(long long tiles, int k_tiles, int max_workers) {
+WorkSplit plan_work_split(long long tiles, int k_tiles, int max_workers, double summing) {
     const long long whole_workers_max = tiles < max_workers ? tiles : max_workers;
     const long long waves = (tiles + whole_workers_max - 1) / whole_workers_max;
     const double cost_whole = static_cast<double>(waves) * k_tiles;
     const double share = static_cast<double>(tiles) * k_tiles / max_workers;
     const double per_tile = static_cast<double>(k_tiles) / (share < 1.0 ? 1.0 : share);   // workers that share a tile, about
-    const double cost_split = share + (share >= 2.0 * k_tiles ? 16.0 : 12.0 * (per_tile < 2.0 ? 2.0 : per_tile));
+    const double cost_split = share + (share >= 2.0 * k_tiles ? summing : 12.0 * (per_tile < 2.0 ? 2.0 : per_tile));
     if (cost_whole <= cost_split) return WorkSplit{cost_whole, static_cast<int>((tiles + waves - 1) / waves), true};   // the fewest workers that need no more waves
     return WorkSplit{cost_split, max_workers, false};
 }
 
 template <int CG, int BN, int STAGES, bool TMA_STORE, int EPI_KB, bool EPI_EX = false, int EPI_WARPS = 0>
-int launch_gemm(DeviceCtx* c, int variant, GemmParams& params, int grid_request, cudaStream_t stream, const char* name) {
+int launch_gemm(DeviceCtx* c, int variant, GemmParams& params, const nvfp4_gemm_config& cf, cudaStream_t stream, const char* name) {
+    const int grid_request = cf.grid;
     using S = GemmSmem<CG, BN, STAGES, TMA_STORE, EPI_KB, 1, EPI_WARPS>;
     auto kernel = gemm_nvfp4_kernel<CG, BN, STAGES, TMA_STORE, EPI_KB, 1, EPI_EX, EPI_WARPS>;
     if (!c->smem_attr_set[variant]) {
@@ -303,13 +305,20 @@ int launch_gemm(DeviceCtx* c, int variant, GemmParams& params, int grid_request,
     if (grid > kMaxCtas) grid = kMaxCtas;
     int workers = grid / CG;
     if (grid_request <= 0) {
-        const WorkSplit split = plan_work_split(params.total_units / params.k_tiles, params.k_tiles, workers);
+        const WorkSplit split = plan_work_split(params.total_units / params.k_tiles, params.k_tiles, workers, kSumming);
         workers = split.workers;
-        if (split.whole_tiles) {
-            params.whole_tiles = 1;
-            params.raster_rows = 0;
-        }
+        params.whole_tiles = split.whole_tiles ? 1 : 0;
+        // Groups of row tiles pay for whole tiles too, where a wave spans several rows and columns of tiles (4096 x 4096 x
+        // 7168 x 4, 117 MB of operands: 179 us, row by row 272; 6144 x 4096 x 7168 x 4: 278, 427).  With fewer the plain order
+        // shares as much, and a worker's neighbouring tiles more (1536 x 6144 x 7168 x 4: 104 us, in groups 107; 200 x 4608 x
+        // 7168 x 4: 18.9, 19.6; 8192 x 128 x 4096 x 4: 17.8, 18.7).  The extended epilogue, which writes row by row itself, gains
+        // from the groups beyond about 93 MB only (to NVFP4: 4096 x 4096 x 7168 x 4 271 -> 204 us, 4096 x 2560 x 7168 x 4, 95 MB,
+        // 164 -> 145; 2304 x 4096 x 7168 x 4, 92 MB, 119 -> 128, 3000 x 7168 x 4096 x 4, 83 MB, 228 -> 252).
+        const double operand_bytes = static_cast<double>(params.L) * (static_cast<double>(params.M) + params.N) * (params.K / 2);
+        if (split.whole_tiles && cf.raster == 0 && (params.tiles_m < 8 || params.tiles_n < 4 || (EPI_EX && operand_bytes < 93e6))) params.raster_rows = 0;
     }
+    params.order_k = params.whole_tiles ? 1 : params.k_tiles;
+    params.order_total = params.whole_tiles ? params.total_units / params.k_tiles : params.total_units;
     if (workers > params.total_units) workers = params.total_units;
     if (workers < 1) workers = 1;
     grid = workers * CG;
@@ -458,8 +467,12 @@ TileChoice choose_tile(int m, int n, int k, int l, int num_sms, const nvfp4_gemm
         const int k_tiles = k / kKPerStage;
         const long long tiles256 = static_cast<long long>((m + 2 * kBM - 1) / (2 * kBM)) * (n / 256) * l;
         const long long tiles128 = static_cast<long long>((m + kBM - 1) / kBM) * (n / 128) * l;
-        const double cost_pair = plan_work_split(tiles256, k_tiles, num_sms / 2).cost + 9.0;
-        const double cost_single = plan_work_split(tiles128, k_tiles, num_sms).cost * 0.9 + 4.5;
+        const double cost_pair = plan_work_split(tiles256, k_tiles, num_sms / 2, kSumming).cost + 9.0;
+        // Single CTAs sum their shared tiles beside more of the whole ones the longer K is: 320 tiles of 128 x 128 evenly
+        // split took 47, 43, 51 and 65 k-tiles' time at 4, 8, 16 and 28 k-tiles, that is 39, 26, 17 and 6 for the summing.
+        // (2048 x 2560 x 7168: 22.6 us so and 25.2 as 80 pair tiles; x 4096: 17.9, 17.3; x 2048: 15.2, 12.4.)
+        const double summing_single = k_tiles < 29 ? 38.0 - 1.2 * k_tiles : 3.0;
+        const double cost_single = plan_work_split(tiles128, k_tiles, num_sms, summing_single).cost * 0.9 + 4.5;
         if (cost_single < cost_pair) cg = 1;
     }
     int bn = cf.tile_n;
@@ -706,27 +719,26 @@ int gemm_impl(const nvfp4_problem* p, const nvfp4_gemm_config* cfg, const nvfp4_
         return launch_gemm_splitk<256, 4, 0, 8>(c, 11, g, stream, "gemm_splitk8_n256_s4");
     }
 
-    const int grid = cf.grid;
     if (epi) {
-        if (cg == 2 && bn == 256) return launch_gemm<2, 256, 5, false, 32, true>(c, 17, g, grid, stream, "gemm_2cta_n256_s5_epilogue");
-        if (cg == 2) return launch_gemm<2, 128, 6, false, 32, true>(c, 18, g, grid, stream, "gemm_2cta_n128_s6_epilogue");
-        if (bn == 256) return launch_gemm<1, 256, 3, false, 48, true>(c, 19, g, grid, stream, "gemm_1cta_n256_s3_epilogue");
-        return launch_gemm<1, 128, 4, false, 64, true>(c, 20, g, grid, stream, "gemm_1cta_n128_s4_epilogue");
+        if (cg == 2 && bn == 256) return launch_gemm<2, 256, 5, false, 32, true>(c, 17, g, cf, stream, "gemm_2cta_n256_s5_epilogue");
+        if (cg == 2) return launch_gemm<2, 128, 6, false, 32, true>(c, 18, g, cf, stream, "gemm_2cta_n128_s6_epilogue");
+        if (bn == 256) return launch_gemm<1, 256, 3, false, 48, true>(c, 19, g, cf, stream, "gemm_1cta_n256_s3_epilogue");
+        return launch_gemm<1, 128, 4, false, 64, true>(c, 20, g, cf, stream, "gemm_1cta_n128_s4_epilogue");
     }
     if (cg == 2) {
-        if (bn == 256 && epilogue == 3) return launch_gemm<2, 256, 4, true, 64>(c, 12, g, grid, stream, "gemm_2cta_n256_s4_tmastore4");
-        if (bn == 256 && epilogue == 2) return launch_gemm<2, 256, 5, true, 32>(c, 4, g, grid, stream, "gemm_2cta_n256_s5_tmastore");
-        if (bn == 256) return launch_gemm<2, 256, 5, false, 32>(c, 5, g, grid, stream, "gemm_2cta_n256_s5_direct");
-        if (epilogue >= 2) return launch_gemm<2, 128, 6, true, 32>(c, 6, g, grid, stream, "gemm_2cta_n128_s6_tmastore");
-        return launch_gemm<2, 128, 6, false, 32>(c, 7, g, grid, stream, "gemm_2cta_n128_s6_direct");
+        if (bn == 256 && epilogue == 3) return launch_gemm<2, 256, 4, true, 64>(c, 12, g, cf, stream, "gemm_2cta_n256_s4_tmastore4");
+        if (bn == 256 && epilogue == 2) return launch_gemm<2, 256, 5, true, 32>(c, 4, g, cf, stream, "gemm_2cta_n256_s5_tmastore");
+        if (bn == 256) return launch_gemm<2, 256, 5, false, 32>(c, 5, g, cf, stream, "gemm_2cta_n256_s5_direct");
+        if (epilogue >= 2) return launch_gemm<2, 128, 6, true, 32>(c, 6, g, cf, stream, "gemm_2cta_n128_s6_tmastore");
+        return launch_gemm<2, 128, 6, false, 32>(c, 7, g, cf, stream, "gemm_2cta_n128_s6_direct");
     }
     // (eight epilogue warps for many tiles of one k-tile: see GemmSmem)
     if (bn == 128 && epilogue >= 2 && g.k_tiles == 1 && g.total_units > 2 * c->num_sms)
-        return launch_gemm<1, 128, 5, true, 32, false, 8>(c, 21, g, grid, stream, "gemm_1cta_n128_s5_tmastore");
-    if (bn == 128 && epilogue >= 2) return launch_gemm<1, 128, 5, true, 32>(c, 0, g, grid, stream, "gemm_1cta_n128_s5_tmastore");
-    if (bn == 128) return launch_gemm<1, 128, 4, false, 64>(c, 1, g, grid, stream, "gemm_1cta_n128_s4_direct");
-    if (epilogue >= 2) return launch_gemm<1, 256, 3, true, 32>(c, 2, g, grid, stream, "gemm_1cta_n256_s3_tmastore");
-    return launch_gemm<1, 256, 3, false, 48>(c, 3, g, grid, stream, "gemm_1cta_n256_s3_direct");
+        return launch_gemm<1, 128, 5, true, 32, false, 8>(c, 21, g, cf, stream, "gemm_1cta_n128_s5_tmastore");
+    if (bn == 128 && epilogue >= 2) return launch_gemm<1, 128, 5, true, 32>(c, 0, g, cf, stream, "gemm_1cta_n128_s5_tmastore");
+    if (bn == 128) return launch_gemm<1, 128, 4, false, 64>(c, 1, g, cf, stream, "gemm_1cta_n128_s4_direct");
+    if (epilogue >= 2) return launch_gemm<1, 256, 3, true, 32>(c, 2, g, cf, stream, "gemm_1cta_n256_s3_tmastore");
+    return launch_gemm<1, 256, 3, false, 48>(c, 3, g, cf, stream, "gemm_1cta_n256_s3_direct");
 }
 }  // namespace
 
@@ -1181,7 +1193,7 @@ int nvfp4_plan_tile_shape(int m, int n, int k, int l, int num_sms, int* cta_grou
 
 int nvfp4_plan_work_split(int64_t tiles, int k_tiles, int max_workers, int* workers, int* whole_tiles) {
     if (tiles < 1 || k_tiles < 1 || max_workers < 1 || !workers || !whole_tiles) return fail(NVFP4_ERR_INVALID_ARGUMENT, "bad work-split query");
-    const WorkSplit split = plan_work_split(tiles, k_tiles, max_workers);
+    const WorkSplit split = plan_work_split(tiles, k_tiles, max_workers, kSumming);
     *workers = split.workers;
     *whole_tiles = split.whole_tiles ? 1 : 0;
     return NVFP4_OK;

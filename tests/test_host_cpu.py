@@ -231,6 +231,38 @@ def test_tile_order_visits_every_output_tile_once(lib, tiles_m, tiles_n, batches
     assert lib.nvfp4_plan_tile(tiles * k_tiles, workers, k_tiles, tiles_m, tiles_n, raster, tiles, ctypes.byref(b), ctypes.byref(r), ctypes.byref(c)) != 0
 
 
+@pytest.mark.parametrize("raster", [0, 1, 8, 16])
+@pytest.mark.parametrize("tiles_m,tiles_n,batches,workers", [(16, 16, 4, 74), (16, 16, 4, 69), (9, 10, 1, 45), (7, 31, 3, 148), (33, 1, 2, 66), (1, 5, 1, 5)])
+def test_whole_tile_order_visits_every_output_tile_once(lib, tiles_m, tiles_n, batches, workers, raster):
+    """Workers that take whole tiles count their ranges in tiles: one unit each.  Tiles at the same place of
+    the workers' ranges are neighbours in the grouped order."""
+    tiles = tiles_m * tiles_n * batches
+    b, r, c = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+    at = []
+    for t in range(tiles):
+        assert lib.nvfp4_plan_tile(tiles, workers, 1, tiles_m, tiles_n, raster, t, ctypes.byref(b), ctypes.byref(r), ctypes.byref(c)) == 0
+        assert 0 <= b.value < batches and 0 <= r.value < tiles_m and 0 <= c.value < tiles_n
+        at.append((b.value, r.value, c.value))
+    assert len(set(at)) == tiles
+    if raster > 1 and tiles >= 2 * workers and workers > tiles_m:
+        begin, end = ctypes.c_int(), ctypes.c_int()
+        first = []
+        for w in range(workers):
+            assert lib.nvfp4_plan_units(tiles, workers, w, ctypes.byref(begin), ctypes.byref(end), None, 1) == 0
+            first.append(at[begin.value])
+        # the first wave: few row blocks and few column tiles, not a pair of its own for every worker
+        assert len({x[:2] for x in first}) <= min(raster, tiles_m) * 2 and len({(x[0], x[2]) for x in first}) <= -(-workers // min(raster, tiles_m)) + 2
+
+
+@pytest.mark.parametrize("m,n,k,l,exp", [(2048, 2560, 7168, 1, (1, 128)), (512, 2560, 7168, 4, (1, 128)),      # 320 small tiles, evenly split: 22.6 us; 80 pair tiles 25.2
+                                         (2048, 2560, 4096, 1, (2, 256)), (512, 2560, 2048, 4, (2, 256)),      # 17.9, 17.3
+                                         (4096, 4096, 7168, 4, (2, 256)), (2048, 4608, 7168, 4, (2, 256))])
+def test_tile_shape_choice_beyond_two_waves(lib, m, n, k, l, exp):
+    cg, bn = ctypes.c_int(), ctypes.c_int()
+    assert lib.nvfp4_plan_tile_shape(m, n, k, l, 148, ctypes.byref(cg), ctypes.byref(bn)) == 0
+    assert (cg.value, bn.value) == exp
+
+
 @pytest.mark.parametrize("resident", [16 * 148, 5 * 148, 2 * 148])
 @pytest.mark.parametrize("step_rows", [4, 16])
 @pytest.mark.parametrize("m,l", [(1, 1), (1, 8), (1, 33), (10, 32), (100, 8), (1000, 8), (7168, 4), (40000, 4), (5, 700), (31, 1500), (1, 65535), (3, 4000)])
